@@ -1037,11 +1037,10 @@ FM_D void collapse_node(const BNode* __restrict__ bnodes, const DpNode* __restri
         e[a] = ex;
         scale[a] = __uint_as_float(ex << 23);
     }
-    uint32_t meta[8], ql[3][8], qh[3][8];
-    uint32_t imask = 0;
+    uint32_t ql[3][8], qh[3][8];
+    uint32_t imask = 0, lmask = 0;
     int int_rank = 0, prim_off = 0;
     for (int s = 0; s < 8; ++s) {
-        meta[s] = 0;
         for (int a = 0; a < 3; ++a) {
             ql[a][s] = 0;
             qh[a][s] = 0;
@@ -1059,13 +1058,12 @@ FM_D void collapse_node(const BNode* __restrict__ bnodes, const DpNode* __restri
         }
         if (!is_leaf[k]) {
             imask |= 1u << s;
-            meta[s] = 0x20u | (uint32_t)(24 + s);   // nonzero marker; traversal uses imask
             const int q = atomicAdd(&counters[2], 1);
             next_frontier[q] = make_int4(ch[k], child_base + int_rank, sroot, 0);
             ++int_rank;
         } else {
             const int cnt = leaf_cnt[k], beg = leaf_beg[k];
-            meta[s] = (((1u << cnt) - 1u) << 5) | (uint32_t)prim_off;
+            lmask |= ((1u << cnt) - 1u) << (3 * s);
             for (int j = 0; j < cnt; ++j) leaf_prim[prim_base + prim_off + j] = pidx[beg + j];
             prim_off += cnt;
         }
@@ -1074,7 +1072,7 @@ FM_D void collapse_node(const BNode* __restrict__ bnodes, const DpNode* __restri
     uint4* np = wnodes + 5 * (size_t)wslot;
     np[0] = make_uint4(__float_as_uint(lo[0]), __float_as_uint(lo[1]), __float_as_uint(lo[2]),
                        e[0] | (e[1] << 8) | (e[2] << 16) | (imask << 24));
-    np[1] = make_uint4(n_int ? (uint32_t)(child_base - sroot) : 0u, (uint32_t)prim_base, pack4(meta), pack4(meta + 4));
+    np[1] = make_uint4(n_int ? (uint32_t)(child_base - sroot) : 0u, (uint32_t)prim_base, lmask, 0u);
     np[2] = make_uint4(pack4(ql[0]), pack4(ql[0] + 4), pack4(ql[1]), pack4(ql[1] + 4));
     np[3] = make_uint4(pack4(ql[2]), pack4(ql[2] + 4), pack4(qh[0]), pack4(qh[0] + 4));
     np[4] = make_uint4(pack4(qh[1]), pack4(qh[1] + 4), pack4(qh[2]), pack4(qh[2] + 4));
@@ -1109,7 +1107,7 @@ __global__ void k_fill_leaf(const int32_t* __restrict__ leaf_prim, int nleaf, co
             if (p < src.num_tris) {
                 const float* v = src.tri_pos + 9 * (size_t)p;
                 a = make_float4(v[0], v[1], v[2], __uint_as_float((uint32_t)p));
-                b = make_float4(v[3], v[4], v[5], 0.0f);
+                b = make_float4(v[3], v[4], v[5], 1.0f);   // a mesh triangle
                 c = make_float4(v[6], v[7], v[8], 0.0f);
             } else if (p < src.num_tris + 2 * src.num_rects) {
                 const int r = (p - src.num_tris) >> 1, h = (p - src.num_tris) & 1;

@@ -35,6 +35,7 @@
 #include "fm_bsdf_grad.cuh"
 #include "fm_path.cuh"
 #include "fm_render.h"
+#include "fm_trace.cuh"
 
 namespace fm {
 
@@ -477,34 +478,53 @@ FM_D unsigned long long global_ns()
     return t;
 }
 
-// Ray kinds of the trace kernel's combined index space [cont | MIS | shadow].
-constexpr int kRayCont = 0, kRayMis = 1, kRayShadow = 2;
-
-// Sets up the traversal of ray `idx` of the combined index space.
-FM_D int begin_ray(const WfState& st, int64_t idx, int64_t nc, int64_t nm, Traversal& t, const DevScene*& Sp,
-                   int& vid)
-{
-    if (idx < nc) {
-        const int slot = st.cont_q[idx];
-        vid = st.view[slot];
-        Sp = st.views[vid].scene;
-        const float4 o4 = st.ro[slot], d4 = st.rd[slot];
-        trav_begin(t, trace_scene(*Sp), f3{o4.x, o4.y, o4.z}, f3{d4.x, d4.y, d4.z}, 0.0f, kRealMax, false);
-        return kRayCont;
+// The rays of the combined index space as a stream (trace_stream): continuation rays by
+// slot, MIS and shadow rays from their queues.
+struct WfRays {
+    const WfState& st;
+    uint32_t nc, ncm;   // continuation rays, continuation + MIS rays
+    FM_D StreamRay load(uint32_t idx) const
+    {
+        StreamRay q;
+        q.tmin = 0.0f;
+        q.tmax = kRealMax;
+        q.any = false;
+        float4 o4, d4;
+        int vid;
+        if (idx < nc) {
+            const int slot = st.cont_q[idx];
+            vid = st.view[slot];
+            o4 = st.ro[slot];
+            d4 = st.rd[slot];
+            st.cont_v[idx] = vid;
+        } else if (idx < ncm) {
+            o4 = st.mis_o[idx - nc];
+            d4 = st.mis_d[idx - nc];
+            vid = __float_as_int(st.mis_a[idx - nc].w);
+        } else {
+            o4 = st.sh_o[idx - ncm];
+            d4 = st.sh_d[idx - ncm];
+            vid = __float_as_int(st.sh_c[idx - ncm].w);
+            q.tmin = kEps;
+            q.tmax = o4.w;
+            q.any = true;
+        }
+        q.scene = st.views[vid].scene;
+        q.o = f3{o4.x, o4.y, o4.z};
+        q.d = f3{d4.x, d4.y, d4.z};
+        return q;
     }
-    if (idx < nc + nm) {
-        const int64_t q = idx - nc;
-        const float4 o4 = st.mis_o[q], d4 = st.mis_d[q];
-        Sp = st.views[__float_as_int(st.mis_a[q].w)].scene;
-        trav_begin(t, trace_scene(*Sp), f3{o4.x, o4.y, o4.z}, f3{d4.x, d4.y, d4.z}, 0.0f, kRealMax, false);
-        return kRayMis;
+    FM_D float tmin(uint32_t, bool any) const { return any ? kEps : 0.0f; }
+    FM_D void finish(uint32_t idx, const Hit& h) const
+    {
+        if (idx < ncm) {
+            float4* out = idx < nc ? st.cont_h + idx : st.mis_h + (idx - nc);
+            *out = make_float4(h.t, __int_as_float(h.prim), h.b1, h.b2);
+        } else {
+            st.sh_h[idx - ncm] = h.prim >= 0 ? 1u : 0u;
+        }
     }
-    const int64_t q = idx - nc - nm;
-    const float4 o4 = st.sh_o[q], d4 = st.sh_d[q];
-    Sp = st.views[__float_as_int(st.sh_c[q].w)].scene;
-    trav_begin(t, trace_scene(*Sp), f3{o4.x, o4.y, o4.z}, f3{d4.x, d4.y, d4.z}, kEps, o4.w, true);
-    return kRayShadow;
-}
+};
 
 // A continuation ray's result: the shading queue the slot goes to by the hit's material
 // class (0 Disney, 1 other materials; 2 and 3 the same for vertices of adjoint renders
@@ -642,87 +662,17 @@ FM_D void finish_shadow(const WfState& st, int64_t q, const DevScene& S, const H
     }
 }
 
-// Traces every queued ray: continuation rays (closest hit), MIS-BSDF rays (closest hit)
-// and shadow rays (occlusion), and stores the results; k_wf_resolve turns them into
-// radiance and shading work.  Warps are persistent over the combined index space: a
-// lane whose query completes takes the next unclaimed ray (one atomic per warp and
-// refill), so lanes do not idle while the warp's slowest traversal finishes, and the
-// loop holds nothing but traversal.
-// Stack entries per thread kept in shared memory by k_wf_trace (the rest in local memory).
-// Measured on the batched workload (trace ms per step, K = 0 / 4 / 8 / 16 entries):
-// 253.2 / 251.9 / 255.9 / 256.5 -- the shared memory taken from the L1 cache that holds
-// the nodes offsets what the stack saves beyond a few entries.
-constexpr int kTraceSmemStack = 4;
-// Rays a warp claims from the combined index space at once (one atomic per claim instead
-// of one per refill; its lanes then take the rays in order).  Within trace_tail rays of the
-// end, warps claim exactly what their lanes need, so that no warp holds back rays while
-// others run dry.
-constexpr unsigned kTraceChunk = 64;
-
+// Traces every queued ray of the combined index space [cont | MIS | shadow]: continuation
+// and MIS-BSDF rays (closest hit) and shadow rays (occlusion), and stores the results;
+// k_wf_resolve turns them into radiance and shading work.  64 registers: three and five
+// blocks of 256 threads per SM traced the 16-scene batch in 32.0 and 35.4 ms against 29.1.
 __global__ void __launch_bounds__(256, 4) k_wf_trace(WfState st)
 {
-    const int64_t nc = st.qc[kQcTraceCont], nm = st.qc[kQcTraceMis], ns = st.qc[kQcTraceShadow];
-    const int64_t total = nc + nm + ns;
-    extern __shared__ uint2 s_stack[];
-    SharedTopStack<kTraceSmemStack> stack;
-    stack.top = s_stack + threadIdx.x;
-    stack.stride = blockDim.x;
-    Traversal t;
-    const DevScene* Sp = nullptr;
-    int vid = 0;
-    int kind = -1;   // ray kind held by this lane, -1 for none
-    int64_t idx = 0;
-    bool exhausted = false;
-    const int lane = threadIdx.x & 31;
-    // the warp's claimed part of the combined index space, [cur, cend) (warp-uniform)
-    unsigned cur = 0, cend = 0;
-    bool chunk = st.trace_tail < total;
+    const uint32_t nc = st.qc[kQcTraceCont], ncm = nc + st.qc[kQcTraceMis];
+    extern __shared__ float4 s_trace[];
     if (threadIdx.x == 0) atomicMin(&st.tspan[0], global_ns());
-    for (;;) {
-        const bool need = kind < 0 && !exhausted;
-        const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (m) {
-            // lanes take rays from the warp's claimed range first, in lane order
-            const unsigned n = (unsigned)__popc(m);
-            const unsigned have = cend - cur;
-            const unsigned r = (unsigned)__popc(m & lanemask_lt());
-            if (have < n) {
-                // claim a new range: a whole chunk while far from the end of the
-                // queues, exactly the lanes' shortfall near it
-                const unsigned take = chunk ? kTraceChunk : n - have;
-                const int leader = __ffs(m) - 1;
-                unsigned base = 0;
-                if (lane == leader) base = atomicAdd(&st.qc[kQcTraceNext], take);
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (chunk && (int64_t)base + st.trace_tail >= total) chunk = false;
-                if (need) idx = r < have ? (int64_t)cur + r : (int64_t)base + (r - have);
-                cur = base + (n - have);
-                cend = base + take;
-            } else {
-                if (need) idx = (int64_t)cur + r;
-                cur += n;
-            }
-            if (need) {
-                if (idx >= total)
-                    exhausted = true;
-                else
-                    kind = begin_ray(st, idx, nc, nm, t, Sp, vid);
-            }
-        }
-        if (__ballot_sync(0xffffffffu, kind >= 0) == 0) break;
-        if (kind >= 0 && trav_step(t, trace_scene(*Sp), stack, st.status)) {
-            const Hit& h = t.hit;
-            if (kind == kRayCont) {
-                st.cont_h[idx] = make_float4(h.t, __int_as_float(h.prim), h.b1, h.b2);
-                st.cont_v[idx] = vid;
-            }
-            else if (kind == kRayMis)
-                st.mis_h[idx - nc] = make_float4(h.t, __int_as_float(h.prim), h.b1, h.b2);
-            else
-                st.sh_h[idx - nc - nm] = h.prim >= 0 ? 1u : 0u;
-            kind = -1;
-        }
-    }
+    trace_stream(WfRays{st, nc, ncm}, ncm + st.qc[kQcTraceShadow], &st.qc[kQcTraceNext], (uint32_t)st.trace_tail, s_trace,
+                 st.status);
     __syncthreads();
     if (threadIdx.x == 0) atomicMax(&st.tspan[1], global_ns());
 }
@@ -1542,7 +1492,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
         st.cap_sh = std::min<int64_t>(st.cap_sh, tune.queue_limit);
     }
     st.views = c->d_views;
-    st.trace_tail = (int64_t)ctx->num_sms * 64 * kTraceChunk;   // 64 resident warps per SM at most
+    st.trace_tail = (int64_t)ctx->num_sms * 64 * 32;   // a warp of rays for each of 64 resident warps per SM
     st.cnt = c->cnt;
     st.status = ctx->d_status;
     if (ADJ) {
@@ -1566,8 +1516,9 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     cudaEventRecord(c->e0, s);
     // one graph body = `iters_per_graph` iterations of prep -> trace -> resolve -> shade
     // (Disney) -> shade (other materials) [-> replay shading] -> logic [-> gradient scatter]
-    const int trace_grid = sms * 16;
-    const size_t trace_smem = sizeof(uint2) * kTraceSmemStack * (size_t)tune.trace_block;
+    // what is resident at 64 registers per thread; more blocks would only find no rays left
+    const int trace_grid = sms * (1024 / tune.trace_block);
+    const size_t trace_smem = kTraceSmemPerThread * (size_t)tune.trace_block;
     const int shade_grid = (int)std::min<int64_t>((pool + tune.shade_block - 1) / tune.shade_block, (int64_t)sms * 32);
     const int logic_grid = (int)std::min<int64_t>((pool + 255) / 256, (int64_t)sms * 32);
     const int resolve_grid = sms * 16;
