@@ -1,33 +1,79 @@
 // C-ABI: contexts, scene release and ray queries (scene creation: fm_scene_build.cu).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <new>
 #include <unordered_map>
 
-#include "fm_bvh.cuh"
 #include "fm_internal.h"
 #include "fm_staging.h"
+#include "fm_trace.cuh"
 
 using namespace fm;
 
 namespace {
 
-__global__ void k_trace(const __grid_constant__ DevScene S, const float* __restrict__ rays, int64_t n,
-                        int32_t* obj_out, float* t_out, uint8_t* occ_out, uint32_t* status)
+constexpr int kQueryBlock = 128, kQueryBlocksPerSm = 8;   // 64 registers per thread
+
+// Large queries: persistent warps over the stream of rays (see trace_stream).  2 M incoherent
+// rays through 1.3 M triangles: 958 -> 412 us against one thread per ray; 1 M occlusion rays
+// through 20 k triangles: 292 -> 154 us.
+__global__ void __launch_bounds__(kQueryBlock, kQueryBlocksPerSm)
+k_trace(const QueryRays q, uint32_t n, uint32_t tail, unsigned* next, uint32_t* status)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(rays) + 2 * i);
-        const float4 b = __ldg(reinterpret_cast<const float4*>(rays) + 2 * i + 1);
-        Hit h;
-        if (occ_out) {
-            occ_out[i] = trace_ray<true>(S, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, b.w, h, status) ? 1 : 0;
-        } else {
-            const bool hit = trace_ray<false>(S, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, b.w, h, status);
-            obj_out[i] = hit ? __ldg(S.prim_obj + h.prim) : -1;
-            t_out[i] = hit ? h.t : __int_as_float(0x7f800000);
-        }
-    }
+    extern __shared__ float4 s_trace[];
+    trace_stream(q, n, next, tail, s_trace, status);
 }
+
+// Queries whose rays are all in flight at once: the launch takes as long as its slowest warp,
+// so every lane keeps its one ray, and a warp holds only per_warp of them when there are
+// fewer rays than lanes (rays of one warp wait for one another's steps).
+__global__ void __launch_bounds__(kQueryBlock, kQueryBlocksPerSm)
+k_trace_short(const QueryRays q, uint32_t n, uint32_t per_warp, uint32_t* status)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t i = (blockIdx.x * (kQueryBlock / 32) + (threadIdx.x >> 5)) * per_warp + lane;
+    if (lane >= per_warp || i >= n) return;
+    const StreamRay r = q.load(i);
+    Hit h;
+    if (r.any)
+        trace_ray<true>(*r.scene, r.o, r.d, r.tmin, r.tmax, h, status);
+    else
+        trace_ray<false>(*r.scene, r.o, r.d, r.tmin, r.tmax, h, status);
+    q.finish(i, h);
+}
+
+}  // namespace
+
+cudaError_t fm::launch_query(cudaStream_t stream, int num_sms, const QueryRays& q, int64_t n, unsigned* next, uint32_t* status)
+{
+    const int64_t warps = (int64_t)num_sms * kQueryBlocksPerSm * (kQueryBlock / 32);
+    if (n <= 32 * warps) {
+        const uint32_t per_warp = (uint32_t)((n + warps - 1) / warps);
+        const int64_t used = (n + per_warp - 1) / per_warp;
+        k_trace_short<<<(int)((used + kQueryBlock / 32 - 1) / (kQueryBlock / 32)), kQueryBlock, 0, stream>>>(q, (uint32_t)n, per_warp, status);
+        return cudaGetLastError();
+    }
+    constexpr int64_t kLaunchRays = (int64_t)1 << 30;   // ray indices are 32-bit within a launch
+    for (int64_t first = 0; first < n; first += kLaunchRays) {
+        if (first > 0) {
+            const cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned), stream);
+            if (e != cudaSuccess) return e;
+        }
+        QueryRays part = q;
+        part.rays += 2 * first;
+        if (part.occ) part.occ += first;
+        if (part.obj) part.obj += first;
+        if (part.t) part.t += first;
+        k_trace<<<num_sms * kQueryBlocksPerSm, kQueryBlock, kTraceSmemPerThread * kQueryBlock, stream>>>(
+            part, (uint32_t)std::min(n - first, kLaunchRays), (uint32_t)(32 * warps), next, status);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+namespace {
 
 fm_status trace_common(fm_ctx* ctx, const fm_scene* sc, const float* rays, int64_t n, int32_t* obj, float* t,
                        uint8_t* occ, int32_t flags)
@@ -57,12 +103,10 @@ fm_status trace_common(fm_ctx* ctx, const fm_scene* sc, const float* rays, int64
             d_t = reinterpret_cast<float*>(p + 4 * (size_t)n);
         }
     }
-    FM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream), "trace");
-    const int block = 128;
-    int64_t grid = (n + block - 1) / block;
-    if (grid > (int64_t)ctx->num_sms * 64) grid = (int64_t)ctx->num_sms * 64;
-    k_trace<<<(int)grid, block, 0, ctx->stream>>>(sc->dev, d_rays, n, d_obj, d_t, d_occ, ctx->d_status);
-    FM_CUDA_TRY(ctx, cudaGetLastError(), "trace launch");
+    // the status word and, in the same allocation, the query's ray counter
+    FM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, 64, ctx->stream), "trace");
+    const QueryRays q{reinterpret_cast<const float4*>(d_rays), sc->d_dev, d_obj, d_t, d_occ};
+    FM_CUDA_TRY(ctx, launch_query(ctx->stream, ctx->num_sms, q, n, ctx->d_status + 8, ctx->d_status), "trace launch");
     if (!dev) {
         if (occ) {
             FM_CUDA_TRY(ctx, cudaMemcpyAsync(occ, d_occ, n, cudaMemcpyDeviceToHost, ctx->stream), "trace d2h");

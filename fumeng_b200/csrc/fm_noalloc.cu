@@ -10,8 +10,8 @@
 // the process exits.
 #include <mutex>
 
-#include "fm_bvh.cuh"
 #include "fm_internal.h"
+#include "fm_trace.cuh"
 
 namespace fm {
 
@@ -45,18 +45,6 @@ fm_status scratch_for_device(fm_ctx* ctx, unsigned char** out)
     return FM_OK;
 }
 
-__global__ void k_trace_closest_staged(const __grid_constant__ DevScene S, const float4* __restrict__ rays, int64_t n,
-                                       int32_t* obj_out, float* t_out, uint32_t* status)
-{
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float4 a = rays[2 * i], b = rays[2 * i + 1];
-        Hit h;
-        const bool hit = trace_ray<false>(S, f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, b.w, h, status);
-        obj_out[i] = hit ? __ldg(S.prim_obj + h.prim) : -1;
-        t_out[i] = hit ? h.t : __int_as_float(0x7f800000);
-    }
-}
-
 }  // namespace
 
 }  // namespace fm
@@ -82,14 +70,12 @@ extern "C" fm_status fm_trace_closest_noalloc(fm_ctx* ctx, const fm_scene* scene
     int32_t* d_obj = reinterpret_cast<int32_t*>(base + kStatusBytes + 32 * (size_t)kNoallocMaxRays);
     float* d_t = reinterpret_cast<float*>(base + kStatusBytes + 36 * (size_t)kNoallocMaxRays);
     cudaStream_t s = ctx->stream;
-    // the staging area keeps the previous call's contents: the status word must start at 0
-    FM_CUDA_TRY(ctx, cudaMemsetAsync(status, 0, sizeof(uint32_t), s), "noalloc status");
+    // the staging area keeps the previous call's contents: the status word and the ray
+    // counter behind it must start at 0
+    FM_CUDA_TRY(ctx, cudaMemsetAsync(status, 0, kStatusBytes, s), "noalloc status");
     FM_CUDA_TRY(ctx, cudaMemcpyAsync(d_rays, rays, 32 * (size_t)n, cudaMemcpyHostToDevice, s), "noalloc h2d");
-    const int block = 128;
-    int64_t grid = (n + block - 1) / block;
-    if (grid > (int64_t)ctx->num_sms * 64) grid = (int64_t)ctx->num_sms * 64;
-    k_trace_closest_staged<<<(int)grid, block, 0, s>>>(scene->dev, d_rays, n, d_obj, d_t, status);
-    FM_CUDA_TRY(ctx, cudaGetLastError(), "noalloc launch");
+    const QueryRays q{d_rays, scene->d_dev, d_obj, d_t, nullptr};
+    FM_CUDA_TRY(ctx, launch_query(s, ctx->num_sms, q, n, status + 32, status), "noalloc launch");
     FM_CUDA_TRY(ctx, cudaMemcpyAsync(obj_id, d_obj, 4 * (size_t)n, cudaMemcpyDeviceToHost, s), "noalloc d2h");
     FM_CUDA_TRY(ctx, cudaMemcpyAsync(t, d_t, 4 * (size_t)n, cudaMemcpyDeviceToHost, s), "noalloc d2h");
     uint32_t hs = 0;

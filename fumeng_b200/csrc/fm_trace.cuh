@@ -1,4 +1,5 @@
-// Warps that traverse a stream of rays: the loop of the wavefront's trace kernel.
+// Warps that traverse a stream of rays: the loop of the wavefront's trace kernel and of large ray
+// queries.
 //
 // The loop is bound by instruction issue, so it is arranged to run every part of a
 // traversal with as many of the warp's lanes as possible:
@@ -169,5 +170,33 @@ FM_D void trace_stream(const Src& src, uint32_t total, unsigned* next, uint32_t 
         }
     }
 }
+
+// The rays of a query as a stream: n x 8 floats (origin, t_min, direction, t_max) against one
+// scene; results as fm_trace_closest / fm_trace_any return them.
+struct QueryRays {
+    const float4* rays;
+    const DevScene* scene;
+    int32_t* obj;
+    float* t;
+    uint8_t* occ;   // null: closest hits
+    FM_D StreamRay load(uint32_t idx) const
+    {
+        const float4 a = __ldg(rays + 2 * (size_t)idx), b = __ldg(rays + 2 * (size_t)idx + 1);
+        return StreamRay{f3{a.x, a.y, a.z}, f3{b.x, b.y, b.z}, a.w, b.w, occ != nullptr, scene};
+    }
+    FM_D float tmin(uint32_t idx, bool) const { return __ldg(&rays[2 * (size_t)idx].w); }
+    FM_D void finish(uint32_t idx, const Hit& h) const
+    {
+        if (occ) {
+            occ[idx] = h.prim >= 0 ? 1 : 0;
+        } else {
+            obj[idx] = h.prim >= 0 ? __ldg(scene->prim_obj + h.prim) : -1;
+            t[idx] = h.prim >= 0 ? h.t : __int_as_float(0x7f800000);
+        }
+    }
+};
+
+// Traces q's n rays; next and status are device words, zero before the launch.
+cudaError_t launch_query(cudaStream_t stream, int num_sms, const QueryRays& q, int64_t n, unsigned* next, uint32_t* status);
 
 }  // namespace fm
