@@ -208,6 +208,7 @@ fm_status megakernel_views(fm_ctx* ctx, std::vector<WfView> views, Counters* cnt
     float4* partial = reinterpret_cast<float4*>(buf + head + views_bytes);
     for (auto& v : views) {
         v.partial = partial;
+        v.partial_f4 = 3;
         partial += 3 * (size_t)v.cfg.width * v.cfg.height * v.nchunks;
     }
     fm_status st = FM_OK;

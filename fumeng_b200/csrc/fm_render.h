@@ -20,7 +20,8 @@ struct WfView {
     int64_t item_base;       // first work item of this view
     int32_t chunk;           // samples per work item
     int32_t nchunks;         // work items per pixel
-    float4* partial;         // [nchunks * npix * 3] (color Kahan sum, albedo sum, normal sum)
+    float4* partial;         // [nchunks * npix * partial_f4] (color Kahan sum[, albedo sum, normal sum])
+    int32_t partial_f4;      // 3, or 1 when the views' albedo and normal images are not wanted
     float* rgb;              // outputs (device)
     float* alb;
     float* nrm;

@@ -105,6 +105,7 @@ struct WfState {
     uint32_t* sh_h;       // ... shadow ray occluded (1) or not (0)
     int64_t cap_cont, cap_mis, cap_sh;
     unsigned* qc;         // kQc* counters
+    int32_t aov;          // some view wants albedo or normal images: asum / nsum are kept
     int64_t trace_tail;   // rays from the end of the trace queues below which warps claim exactly what they need
     // trace kernel span of the current iteration (earliest block start, latest block
     // end, device global timer in ns) and the sum of the spans so far
@@ -748,6 +749,17 @@ FM_D void kahan_add4(float4& sum, float4& c, f3 x)
     sum.z = tz;
 }
 
+// The Kahan sums of the slot's item over its first `done` samples (nothing is stored before
+// the first).
+FM_D void item_sums(const WfState& st, int slot, int done, float4& sum, float4& cmp)
+{
+    sum = cmp = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (done > 0) {
+        sum = st.isum[slot];
+        cmp = st.icomp[slot];
+    }
+}
+
 FM_D int item_samples(const WfView& V, int chunk_index)
 {
     const int first = chunk_index * V.chunk;
@@ -847,7 +859,7 @@ FM_D void shade_vertices(const WfState& st)
                 D[4] = make_float4(h.u, h.v, 0.0f, 0.0f);
                 st.vg[2 * (size_t)slot] = st.vg[2 * (size_t)slot + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-            if (depth == 1 && !replay) {
+            if (depth == 1 && !replay && st.aov) {
                 const f3 al = bsdf_albedo(b);
                 float4 as = st.asum[slot], ns = st.nsum[slot];
                 as.x += al.x; as.y += al.y; as.z += al.z;
@@ -1113,13 +1125,14 @@ __global__ void __launch_bounds__(256, 6) k_wf_logic(WfState st)
                 const int vid = st.view[slot];
                 const WfView& V = st.views[vid];
                 st.lp[slot] = make_float4(col.x, col.y, col.z, 0.0f);
-                float4 sum = st.isum[slot], cmp = st.icomp[slot];
+                s_k = st.k[slot];
+                float4 sum, cmp;
+                item_sums(st, slot, s_k, sum, cmp);
                 kahan_add4(sum, cmp, col);
                 st.isum[slot] = sum;
                 st.icomp[slot] = cmp;
                 s_vid = vid;
                 s_local = item - V.item_base;
-                s_k = st.k[slot];
                 s_flags = kReplay;
                 enqueue_cont = true;
             } else {
@@ -1133,17 +1146,22 @@ __global__ void __launch_bounds__(256, 6) k_wf_logic(WfState st)
                 }
                 ++n_paths;
                 if (!isfinite(col.x) || !isfinite(col.y) || !isfinite(col.z)) ++n_nans;
-                float4 sum = st.isum[slot], cmp = st.icomp[slot];
+                const int k = st.k[slot];
+                float4 sum, cmp;
+                // the primal pass has added an adjoint render's sample already
+                item_sums(st, slot, ADJ ? k + 1 : k, sum, cmp);
                 if (!ADJ) kahan_add4(sum, cmp, clamp_sample(V.cfg, col));
-                const int kdone = st.k[slot] + 1;
+                const int kdone = k + 1;
                 const int64_t local = item - V.item_base;
                 const int npix = V.cfg.width * V.cfg.height;
                 const int chunk_index = (int)(local / npix);
                 if (kdone >= item_samples(V, chunk_index)) {
-                    float4* P = V.partial + 3 * (size_t)local;
+                    float4* P = V.partial + V.partial_f4 * (size_t)local;
                     P[0] = sum;
-                    P[1] = st.asum[slot];
-                    P[2] = st.nsum[slot];
+                    if (st.aov) {
+                        P[1] = st.asum[slot];
+                        P[2] = st.nsum[slot];
+                    }
                     need_new = true;
                 } else {
                     st.isum[slot] = sum;
@@ -1174,11 +1192,7 @@ __global__ void __launch_bounds__(256, 6) k_wf_logic(WfState st)
                     st.item[slot] = it;
                     st.view[slot] = vid;
                     st.k[slot] = 0;
-                    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    st.isum[slot] = z;
-                    st.icomp[slot] = z;
-                    st.asum[slot] = z;
-                    st.nsum[slot] = z;
+                    if (st.aov) st.asum[slot] = st.nsum[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     s_vid = vid;
                     s_local = it - V.item_base;
                     s_k = 0;
@@ -1242,11 +1256,14 @@ __global__ void k_wf_reduce(WfView V)
         float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f), c = s;
         f3 a = mk(0.0f), n = mk(0.0f);
         for (int ch = 0; ch < V.nchunks; ++ch) {
-            const float4* P = V.partial + 3 * ((size_t)ch * npix + p);
-            const float4 x = P[0], y = P[1], z = P[2];
+            const float4* P = V.partial + V.partial_f4 * ((size_t)ch * npix + p);
+            const float4 x = P[0];
             kahan_add4(s, c, f3{x.x, x.y, x.z});
-            a += f3{y.x, y.y, y.z};
-            n += f3{z.x, z.y, z.z};
+            if (V.alb || V.nrm) {
+                const float4 y = P[1], z = P[2];
+                a += f3{y.x, y.y, y.z};
+                n += f3{z.x, z.y, z.z};
+            }
         }
         const float inv = 1.0f / (float)V.cfg.spp;
         st3(V.rgb + 3 * (size_t)p, f3{s.x, s.y, s.z} * inv);
@@ -1447,6 +1464,10 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     // samples per work item: aim for ~4 items per path slot over the whole job
     double total_samples = 0.0;
     int max_lights = 1, max_dl = 1;
+    // albedo and normal sums are kept, and their partial sums written, only when asked for
+    // (they are a third of a path's state traffic)
+    bool aov = false;
+    for (const auto& v : views) aov = aov || v.alb || v.nrm;
     for (const auto& v : views) {
         total_samples += (double)v.cfg.width * v.cfg.height * v.cfg.spp;
         max_dl = std::max(max_dl, v.cfg.direct_loop);
@@ -1463,7 +1484,8 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
         v.item_base = item_base;
         const int64_t npix = (int64_t)v.cfg.width * v.cfg.height;
         item_base += npix * v.nchunks;
-        partial_f4 += 3 * npix * v.nchunks;
+        v.partial_f4 = aov ? 3 : 1;
+        partial_f4 += v.partial_f4 * npix * v.nchunks;
     }
     WfCache* c = nullptr;
     fm_status result = wf_cache_reserve(ctx, ADJ, pool, pool * max_dl, pool * max_dl * (int64_t)max_lights, partial_f4,
@@ -1473,7 +1495,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
         float4* p = c->partial;
         for (auto& v : views) {
             v.partial = p;
-            p += 3 * (int64_t)v.cfg.width * v.cfg.height * v.nchunks;
+            p += v.partial_f4 * (int64_t)v.cfg.width * v.cfg.height * v.nchunks;
         }
     }
     // the launch state: the workspace's buffers, this call's sizes
@@ -1481,6 +1503,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     std::memcpy(&st, &c->bufs, sizeof(st));
     st.pool = pool;
     st.nviews = (int32_t)views.size();
+    st.aov = aov ? 1 : 0;
     st.total_items = item_base;
     st.cap_cont = pool;
     st.cap_mis = pool * max_dl;
