@@ -492,7 +492,7 @@ def main():
     alg_bytes = totals["closest"] * closest_b + totals["shadow"] * shadow_b
     peak, peak_kind = measured_peak_hbm()
     achieved = alg_bytes / (totals["trace_ms"] / 1e3) / 1e9 if totals["trace_ms"] > 0 else None
-    # six launches per wavefront iteration (prep, trace, resolve, two shade kernels,
+    # six launches per wavefront iteration (trace, two resolve kernels, two shade kernels,
     # logic), one loop-condition kernel per graph body of iters_per_graph iterations,
     # and per step one init, one counter copy and one reduce per view
     it = tuning.iters_per_graph
