@@ -94,57 +94,101 @@ __global__ void k_to_u8(const float* __restrict__ src, uint8_t* __restrict__ dst
     }
 }
 
+// What a tap of the a-trous filter reads, per pixel: the compressed colour t(c) = c / (1 + c)
+// per channel with the colour's red, its green and blue, the unit normal and the albedo.
+// 56 B in four loads.  Computed in every tap from the images as they are, the same values
+// cost six divisions, a square root and nine 4-byte loads 12 bytes apart per tap.
+struct DenoiseIn {
+    const float4* t;   // t(c).xyz | c.x
+    const float2* c;   // c.y, c.z
+    const float4* n;   // unit normal (zero stays zero)
+    const float4* a;   // albedo
+};
+
+// |v|^2 and a . b with their multiply-adds written out, so that the 8-bit images do not
+// depend on how the compiler contracts the sums.
+FM_D float square(f3 v) { return fmaf(v.z, v.z, fmaf(v.x, v.x, __fmul_rn(v.y, v.y))); }
+FM_D float dot_fma(f3 a, f3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, __fmul_rn(a.x, b.x))); }
+
+FM_D f3 compress(f3 c)
+{
+    return f3{c.x / (1.0f + fmaxf(c.x, 0.0f)), c.y / (1.0f + fmaxf(c.y, 0.0f)), c.z / (1.0f + fmaxf(c.z, 0.0f))};
+}
+
+// A colour's records.  A colour that is not finite is never averaged into another pixel: its
+// t.x is NaN, which makes every weight computed from it fail the test of a tap.
+FM_D void put_colour(float4* t, float2* c, int64_t p, f3 v)
+{
+    const f3 u = compress(v);
+    t[p] = make_float4(isfinite(v.x + v.y + v.z) ? u.x : __int_as_float(0x7fffffff), u.y, u.z, v.x);
+    c[p] = make_float2(v.y, v.z);
+}
+
+__global__ void k_denoise_pack(const float* __restrict__ rgb, const float* __restrict__ alb, const float* __restrict__ nrm,
+                               int64_t npix, float4* t, float2* c, float4* n, float4* a)
+{
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x) {
+        put_colour(t, c, p, f3{rgb[3 * p], rgb[3 * p + 1], rgb[3 * p + 2]});
+        f3 np = f3{nrm[3 * p], nrm[3 * p + 1], nrm[3 * p + 2]};
+        const float nl = sqrtf(square(np));
+        np = nl > 0.0f ? np / nl : np;
+        n[p] = make_float4(np.x, np.y, np.z, 0.0f);
+        a[p] = make_float4(alb[3 * p], alb[3 * p + 1], alb[3 * p + 2], 0.0f);
+    }
+}
+
 // One pass of the edge-avoiding a-trous filter at tap distance `step` (pixels).
 // Weights: B3-spline h(dx) h(dy) with h = (1, 4, 6, 4, 1) / 16, times
-//   exp(-|t(c_q) - t(c_p)|^2 / sc^2)          colour, t(c) = c / (1 + c) per channel
+//   exp(-|t(c_q) - t(c_p)|^2 / sc^2)          colour; inv_sc2 = 1 / sc^2, a power of two
 //   exp(-max(0, 1 - n_p . n_q) / sn^2)         normal (unit-normalised AOV means)
 //   exp(-|a_q - a_p|^2 / sa^2)                 albedo
-// with the colour scale halved at every pass (the finer detail has been removed).
-__global__ void k_atrous(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ alb,
-                         const float* __restrict__ nrm, int w, int h, int step, float sc, float sn, float sa)
+// with the colour scale halved at every pass (the finer detail has been removed).  The
+// last pass (rgb set) writes the plain image, the others the next pass's records.  Blocks
+// are 32 x 8 pixels, so that the taps of the first passes are in the L1 cache.
+// Bound by issue slots (about 70 instructions per tap, two of them IEEE divisions that
+// the results depend on); 1920x1080: 418 -> 188 us per pass.
+__global__ void __launch_bounds__(256) k_atrous(DenoiseIn in, int w, int h, int step, float inv_sc2, float sn, float sa,
+                                                float4* __restrict__ t_out, float2* __restrict__ c_out,
+                                                float* __restrict__ rgb)
 {
     const float hk[5] = {1.0f / 16.0f, 4.0f / 16.0f, 6.0f / 16.0f, 4.0f / 16.0f, 1.0f / 16.0f};
-    const int64_t npix = (int64_t)w * h;
-    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npix; p += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(p % w), y = (int)(p / w);
-        const f3 cp = f3{in[3 * p], in[3 * p + 1], in[3 * p + 2]};
-        const f3 tp = f3{cp.x / (1.0f + fmaxf(cp.x, 0.0f)), cp.y / (1.0f + fmaxf(cp.y, 0.0f)),
-                         cp.z / (1.0f + fmaxf(cp.z, 0.0f))};
-        f3 np = f3{nrm[3 * p], nrm[3 * p + 1], nrm[3 * p + 2]};
-        const float nl = length(np);
-        np = nl > 0.0f ? np / nl : np;
-        const f3 ap = f3{alb[3 * p], alb[3 * p + 1], alb[3 * p + 2]};
-        f3 sum = mk(0.0f);
-        float wsum = 0.0f;
-        for (int dy = -2; dy <= 2; ++dy) {
-            const int yy = y + dy * step;
-            if (yy < 0 || yy >= h) continue;
-            for (int dx = -2; dx <= 2; ++dx) {
-                const int xx = x + dx * step;
-                if (xx < 0 || xx >= w) continue;
-                const int64_t q = (int64_t)yy * w + xx;
-                const f3 cq = f3{in[3 * q], in[3 * q + 1], in[3 * q + 2]};
-                const f3 tq = f3{cq.x / (1.0f + fmaxf(cq.x, 0.0f)), cq.y / (1.0f + fmaxf(cq.y, 0.0f)),
-                                 cq.z / (1.0f + fmaxf(cq.z, 0.0f))};
-                f3 nq = f3{nrm[3 * q], nrm[3 * q + 1], nrm[3 * q + 2]};
-                const float ql = length(nq);
-                nq = ql > 0.0f ? nq / ql : nq;
-                const f3 aq = f3{alb[3 * q], alb[3 * q + 1], alb[3 * q + 2]};
-                const f3 dc = tq - tp, da = aq - ap;
-                const float wc = __expf(-dot(dc, dc) / (sc * sc));
-                const float wn = __expf(-fmaxf(0.0f, 1.0f - dot(np, nq)) / (sn * sn));
-                const float wa = __expf(-dot(da, da) / (sa * sa));
-                const float wt = hk[dx + 2] * hk[dy + 2] * wc * wn * wa;
-                if (!(wt > 0.0f) || !isfinite(cq.x + cq.y + cq.z)) continue;
-                sum += cq * wt;
-                wsum += wt;
-            }
+    const int tiles_x = (w + 31) / 32;
+    const int x = (int)(blockIdx.x % tiles_x) * 32 + (threadIdx.x & 31), y = (int)(blockIdx.x / tiles_x) * 8 + (threadIdx.x >> 5);
+    if (x >= w || y >= h) return;
+    const int64_t p = (int64_t)y * w + x;
+    const float4 t4 = __ldg(in.t + p), n4 = __ldg(in.n + p), a4 = __ldg(in.a + p);
+    const float2 c2 = __ldg(in.c + p);
+    const f3 cp = f3{t4.w, c2.x, c2.y}, np = f3{n4.x, n4.y, n4.z}, ap = f3{a4.x, a4.y, a4.z};
+    const f3 tp = t4.x == t4.x ? f3{t4.x, t4.y, t4.z} : compress(cp);
+    f3 sum = mk(0.0f);
+    float wsum = 0.0f;
+#pragma unroll 1
+    for (int dy = -2; dy <= 2; ++dy) {
+        const int yy = y + dy * step;
+        if (yy < 0 || yy >= h) continue;
+#pragma unroll
+        for (int dx = -2; dx <= 2; ++dx) {
+            const int xx = x + dx * step;
+            if (xx < 0 || xx >= w) continue;
+            const int64_t q = (int64_t)yy * w + xx;
+            const float4 tq4 = __ldg(in.t + q), nq4 = __ldg(in.n + q), aq4 = __ldg(in.a + q);
+            const float2 cq2 = __ldg(in.c + q);
+            const f3 tq = f3{tq4.x, tq4.y, tq4.z}, nq = f3{nq4.x, nq4.y, nq4.z}, aq = f3{aq4.x, aq4.y, aq4.z};
+            const f3 dc = tq - tp, da = aq - ap;
+            const float wc = __expf(-square(dc) * inv_sc2);
+            const float wn = __expf(-fmaxf(0.0f, __fsub_rn(1.0f, dot_fma(np, nq))) / (sn * sn));
+            const float wa = __expf(-square(da) / (sa * sa));
+            const float wt = hk[dx + 2] * hk[dy + 2] * wc * wn * wa;
+            if (!(wt > 0.0f)) continue;
+            sum += f3{tq4.w, cq2.x, cq2.y} * wt;
+            wsum += wt;
         }
-        const f3 r = wsum > 0.0f ? sum / wsum : cp;
-        out[3 * p] = r.x;
-        out[3 * p + 1] = r.y;
-        out[3 * p + 2] = r.z;
     }
+    const f3 r = wsum > 0.0f ? sum / wsum : cp;
+    if (rgb)
+        st3(rgb + 3 * p, r);
+    else
+        put_colour(t_out, c_out, p, r);
 }
 
 }  // namespace
@@ -179,9 +223,10 @@ extern "C" fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, 
     const bool dev = (flags & FM_FLAG_DEVICE_PTRS) != 0;
     const int64_t n = (int64_t)width * height * 3;
     const size_t fbytes = (size_t)n * sizeof(float);
-    // device copies when the caller's buffers are host memory, a ping-pong image for the
-    // denoiser, and the 8-bit outputs
-    const size_t need = (dev ? 0 : 3 * fbytes) + (denoise ? fbytes : 0) + (dev ? 0 : 3 * (size_t)n) + 1024;
+    // device copies when the caller's buffers are host memory, the denoiser's records (two
+    // sets of colours, one of guides: 80 B per pixel), and the 8-bit outputs
+    const size_t npix = (size_t)width * height;
+    const size_t need = (dev ? 0 : 3 * fbytes) + (denoise ? 80 * npix : 0) + (dev ? 0 : 3 * (size_t)n) + 4096;
     char* tmp = nullptr;
     FM_CUDA_TRY(ctx, cudaMallocAsync((void**)&tmp, need, s), "postprocess alloc");
     char* q = tmp;
@@ -208,7 +253,16 @@ extern "C" fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, 
         d_alb8 = albedo8 && albedo ? reinterpret_cast<uint8_t*>(take((size_t)n)) : nullptr;
         d_nrm8 = normal8 && normal ? reinterpret_cast<uint8_t*>(take((size_t)n)) : nullptr;
     }
-    float* pong = denoise ? reinterpret_cast<float*>(take(fbytes)) : nullptr;
+    float4 *den_t[2] = {}, *den_n = nullptr, *den_a = nullptr;
+    float2* den_c[2] = {};
+    if (denoise) {
+        for (int k = 0; k < 2; ++k) {
+            den_t[k] = reinterpret_cast<float4*>(take(16 * npix));
+            den_c[k] = reinterpret_cast<float2*>(take(8 * npix));
+        }
+        den_n = reinterpret_cast<float4*>(take(16 * npix));
+        den_a = reinterpret_cast<float4*>(take(16 * npix));
+    }
     const int block = 256;
     const int grid = (int)std::min<int64_t>((n + block - 1) / block, (int64_t)ctx->num_sms * 16);
     const int pgrid = (int)std::min<int64_t>(((int64_t)width * height + block - 1) / block, (int64_t)ctx->num_sms * 16);
@@ -220,17 +274,17 @@ extern "C" fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, 
             e = cudaGetLastError();
         }
         if (i < num_steps && e == cudaSuccess) {
-            // five a-trous passes, ping-ponging between the image and `pong`; an odd number
-            // of passes ends in `pong`, which is copied back
-            float* src = d_rgb;
-            float* dst = pong;
-            for (int k = 0; k < 5 && e == cudaSuccess; ++k) {
-                k_atrous<<<pgrid, block, 0, s>>>(src, dst, d_alb, d_nrm, width, height, 1 << k, 0.5f / (float)(1 << k),
-                                                 0.35f, 0.1f);
-                e = cudaGetLastError();
-                std::swap(src, dst);
+            // five a-trous passes between two sets of colour records; the last one writes
+            // the image
+            k_denoise_pack<<<pgrid, block, 0, s>>>(d_rgb, d_alb, d_nrm, (int64_t)npix, den_t[0], den_c[0], den_n, den_a);
+            const int tiles = ((width + 31) / 32) * ((height + 7) / 8);
+            for (int k = 0; k < 5; ++k) {
+                const DenoiseIn in{den_t[k & 1], den_c[k & 1], den_n, den_a};
+                const float sc = 0.5f / (float)(1 << k);
+                k_atrous<<<tiles, 256, 0, s>>>(in, width, height, 1 << k, 1.0f / (sc * sc), 0.35f, 0.1f,
+                                               den_t[(k + 1) & 1], den_c[(k + 1) & 1], k == 4 ? d_rgb : nullptr);
             }
-            if (e == cudaSuccess && src != d_rgb) e = cudaMemcpyAsync(d_rgb, src, fbytes, cudaMemcpyDeviceToDevice, s);
+            e = cudaGetLastError();
         }
         first = i + 1;
     }
