@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "fm_render.h"
+#include "fm_staging.h"
 
 namespace fm {
 
@@ -72,8 +73,7 @@ extern "C" fm_status fm_scene_update_texture(fm_ctx* ctx, fm_scene* scene, int32
         if (!(flags & FM_FLAG_DEVICE_PTRS)) {
             float* staged = a.get<float>(3 * n);
             if (!staged) return set_error(ctx, FM_ERR_OOM, "update_texture: staging allocation failed");
-            FM_CUDA_TRY(ctx, cudaMemcpyAsync(staged, texels, 3 * n * sizeof(float), cudaMemcpyHostToDevice, s),
-                        "update_texture h2d");
+            FM_CUDA_TRY(ctx, copy_in(ctx, s, {InCopy{staged, texels, 3 * n * sizeof(float)}}), "update_texture h2d");
             src = staged;
         }
         launch_rgb_to_texels(s, src, const_cast<float4*>(t.texels), n, ctx->num_sms);
@@ -177,6 +177,7 @@ extern "C" fm_status fm_render_adjoint(fm_ctx* ctx, const fm_scene* scene, int32
         FM_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), s), "render_adjoint");
         // per-view dLoss/dI inputs and image outputs
         std::vector<WfView> views((size_t)n);
+        std::vector<InCopy> inputs;
         for (int32_t i = 0; i < n; ++i) {
             img_floats[i] = (size_t)out_width(params[i]) * out_height(params[i]) * 3;
             const size_t bytes = img_floats[i] * sizeof(float);
@@ -185,8 +186,7 @@ extern "C" fm_status fm_render_adjoint(fm_ctx* ctx, const fm_scene* scene, int32
             } else {
                 drgb_in[i] = a.get<float>(img_floats[i]);
                 if (!drgb_in[i]) return oom();
-                FM_CUDA_TRY(ctx, cudaMemcpyAsync(drgb_in[i], d_rgb[i], bytes, cudaMemcpyHostToDevice, s),
-                            "render_adjoint h2d");
+                inputs.push_back(InCopy{drgb_in[i], d_rgb[i], bytes});
             }
             // the wavefront always writes a primal image; scratch when none is wanted
             if (dev && rgb && rgb[i]) {
@@ -204,6 +204,7 @@ extern "C" fm_status fm_render_adjoint(fm_ctx* ctx, const fm_scene* scene, int32
             v.rgb = rgb_out[i];
             v.drgb = drgb_in[i];
         }
+        FM_CUDA_TRY(ctx, copy_in(ctx, s, inputs), "render_adjoint h2d");
         // the env light's importance densities depend on every texel through their row
         // and map sums: score sums per row and in total, spread after the render
         const int env_tex = scene->dev.env_light >= 0 ? scene->dev.env.tex : -1;
@@ -230,27 +231,15 @@ extern "C" fm_status fm_render_adjoint(fm_ctx* ctx, const fm_scene* scene, int32
         if (result == FM_OK && env_row)
             result = env_grad_finalize(ctx, scene->textures[env_tex], env_row, env_total, dtex[env_tex]);
         if (result == FM_OK && !dev) {
-            // results back to the host: images, then gradients added into the caller's buffers
+            // results back to the host: images, and gradients added into the caller's buffers
+            std::vector<OutCopy> out;
             for (int32_t i = 0; i < n; ++i)
-                if (rgb && rgb[i])
-                    cudaMemcpyAsync(rgb[i], rgb_out[i], img_floats[i] * sizeof(float), cudaMemcpyDeviceToHost, s);
-            for (int t = 0; t < nt; ++t) {
-                if (!dtex[t]) continue;
-                const size_t cnt = (size_t)scene->textures[t].w * scene->textures[t].h * 3;
-                std::vector<double> h(cnt);
-                FM_CUDA_TRY(ctx, cudaMemcpyAsync(h.data(), dtex[t], cnt * sizeof(double), cudaMemcpyDeviceToHost, s),
-                            "render_adjoint d2h");
-                FM_CUDA_TRY(ctx, cudaStreamSynchronize(s), "render_adjoint");
-                double* user = grads->texture_grads[t];
-                for (size_t q = 0; q < cnt; ++q) user[q] += h[q];
-            }
-            if (dmat) {
-                std::vector<double> h((size_t)nm * kGradParams);
-                FM_CUDA_TRY(ctx, cudaMemcpyAsync(h.data(), dmat, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s),
-                            "render_adjoint d2h");
-                FM_CUDA_TRY(ctx, cudaStreamSynchronize(s), "render_adjoint");
-                for (size_t q = 0; q < h.size(); ++q) grads->material_grads[q] += h[q];
-            }
+                if (rgb && rgb[i]) out.push_back(OutCopy{rgb[i], rgb_out[i], img_floats[i] * sizeof(float)});
+            for (int t = 0; t < nt; ++t)
+                if (dtex[t]) out.push_back(OutCopy{grads->texture_grads[t], dtex[t], tex_n[t] * sizeof(double), true});
+            if (dmat)
+                out.push_back(OutCopy{grads->material_grads, dmat, (size_t)nm * kGradParams * sizeof(double), true});
+            FM_CUDA_TRY(ctx, copy_results(ctx, s, out), "render_adjoint d2h");
         }
         cudaMemcpyAsync(&hc, d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s);
         cudaMemcpyAsync(&hs, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);

@@ -94,7 +94,7 @@ fm_status trace_common(fm_ctx* ctx, const fm_scene* sc, const float* rays, int64
         FM_CUDA_TRY(ctx, cudaMallocAsync(&tmp, bytes, ctx->stream), "trace alloc");
         char* p = static_cast<char*>(tmp);
         d_rays = reinterpret_cast<float*>(p);
-        FM_CUDA_TRY(ctx, cudaMemcpyAsync(p, rays, 32 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream), "trace h2d");
+        FM_CUDA_TRY(ctx, copy_in(ctx, ctx->stream, {InCopy{p, rays, 32 * (size_t)n}}), "trace h2d");
         p += 32 * (size_t)n;
         if (occ) {
             d_occ = reinterpret_cast<uint8_t*>(p);
@@ -108,12 +108,10 @@ fm_status trace_common(fm_ctx* ctx, const fm_scene* sc, const float* rays, int64
     const QueryRays q{reinterpret_cast<const float4*>(d_rays), sc->d_dev, d_obj, d_t, d_occ};
     FM_CUDA_TRY(ctx, launch_query(ctx->stream, ctx->num_sms, q, n, ctx->d_status + 8, ctx->d_status), "trace launch");
     if (!dev) {
-        if (occ) {
-            FM_CUDA_TRY(ctx, cudaMemcpyAsync(occ, d_occ, n, cudaMemcpyDeviceToHost, ctx->stream), "trace d2h");
-        } else {
-            FM_CUDA_TRY(ctx, cudaMemcpyAsync(obj, d_obj, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
-            FM_CUDA_TRY(ctx, cudaMemcpyAsync(t, d_t, 4 * (size_t)n, cudaMemcpyDeviceToHost, ctx->stream), "d2h");
-        }
+        if (occ)
+            FM_CUDA_TRY(ctx, copy_results(ctx, ctx->stream, {OutCopy{occ, d_occ, (size_t)n}}), "trace d2h");
+        else
+            FM_CUDA_TRY(ctx, copy_results(ctx, ctx->stream, {OutCopy{obj, d_obj, 4 * (size_t)n}, OutCopy{t, d_t, 4 * (size_t)n}}), "trace d2h");
         FM_CUDA_TRY(ctx, cudaFreeAsync(tmp, ctx->stream), "trace free");
     }
     uint32_t status = 0;

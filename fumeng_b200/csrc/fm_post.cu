@@ -24,6 +24,7 @@
 
 #include "fm_common.cuh"
 #include "fm_internal.h"
+#include "fm_staging.h"
 
 namespace fm {
 
@@ -244,9 +245,10 @@ extern "C" fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, 
         d_rgb = reinterpret_cast<float*>(take(fbytes));
         float* a = albedo ? reinterpret_cast<float*>(take(fbytes)) : nullptr;
         float* nn = normal ? reinterpret_cast<float*>(take(fbytes)) : nullptr;
-        e = cudaMemcpyAsync(d_rgb, rgb, fbytes, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess && a) e = cudaMemcpyAsync(a, albedo, fbytes, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess && nn) e = cudaMemcpyAsync(nn, normal, fbytes, cudaMemcpyHostToDevice, s);
+        std::vector<InCopy> in{InCopy{d_rgb, rgb, fbytes}};
+        if (a) in.push_back(InCopy{a, albedo, fbytes});
+        if (nn) in.push_back(InCopy{nn, normal, fbytes});
+        e = copy_in(ctx, s, in);
         d_alb = a;
         d_nrm = nn;
         d_rgb8 = rgb8 ? reinterpret_cast<uint8_t*>(take((size_t)n)) : nullptr;
@@ -301,10 +303,11 @@ extern "C" fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, 
         e = cudaGetLastError();
     }
     if (!dev && e == cudaSuccess) {
-        e = cudaMemcpyAsync(rgb, d_rgb, fbytes, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && d_rgb8) e = cudaMemcpyAsync(rgb8, d_rgb8, (size_t)n, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && d_alb8) e = cudaMemcpyAsync(albedo8, d_alb8, (size_t)n, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess && d_nrm8) e = cudaMemcpyAsync(normal8, d_nrm8, (size_t)n, cudaMemcpyDeviceToHost, s);
+        std::vector<OutCopy> out{OutCopy{rgb, d_rgb, fbytes}};
+        if (d_rgb8) out.push_back(OutCopy{rgb8, d_rgb8, (size_t)n});
+        if (d_alb8) out.push_back(OutCopy{albedo8, d_alb8, (size_t)n});
+        if (d_nrm8) out.push_back(OutCopy{normal8, d_nrm8, (size_t)n});
+        e = copy_results(ctx, s, out);
     }
     cudaFreeAsync(tmp, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);

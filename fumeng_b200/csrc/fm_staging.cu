@@ -231,6 +231,71 @@ void Stager::close()
     used = kStageChunk;
 }
 
+namespace {
+
+// dst[i] += src[i], split over the copy threads.
+void add_doubles(fm_ctx* ctx, double* dst, const double* src, size_t n)
+{
+    constexpr size_t kSlice = size_t(1) << 15;
+    const int tasks = (int)((n + kSlice - 1) / kSlice);
+    host_parallel(ctx, tasks, [&](int i) {
+        const size_t end = std::min(n, ((size_t)i + 1) * kSlice);
+        for (size_t q = (size_t)i * kSlice; q < end; ++q) dst[q] += src[q];
+    });
+}
+
+}  // namespace
+
+cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies)
+{
+    size_t total = 0;
+    for (const InCopy& c : copies) total += c.bytes;
+    if (total < kRingBytes) {
+        for (const InCopy& c : copies) {
+            const cudaError_t e = cudaMemcpyAsync(c.dst_dev, c.src_host, c.bytes, cudaMemcpyHostToDevice, s);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    const cudaError_t e = staging_ensure(ctx);
+    if (e != cudaSuccess) return e;
+    Stager stager(ctx, s);
+    for (const InCopy& c : copies) stager.put(c.dst_dev, c.src_host, c.bytes);
+    stager.close();
+    return stager.err;
+}
+
+cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies)
+{
+    size_t total = 0, added = 0;
+    for (const OutCopy& c : copies) {
+        total += c.bytes;
+        if (c.add) added += c.bytes / sizeof(double);
+    }
+    if (total >= kRingBytes) return copy_out(ctx, s, copies);
+    std::vector<double> sums(added);
+    size_t at = 0;
+    for (const OutCopy& c : copies) {
+        void* dst = c.dst_host;
+        if (c.add) {
+            dst = sums.data() + at;
+            at += c.bytes / sizeof(double);
+        }
+        const cudaError_t e = cudaMemcpyAsync(dst, c.src_dev, c.bytes, cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) return e;
+    }
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return e;
+    at = 0;
+    for (const OutCopy& c : copies) {
+        if (!c.add) continue;
+        double* dst = static_cast<double*>(c.dst_host);
+        for (size_t q = 0; q < c.bytes / sizeof(double); ++q) dst[q] += sums[at + q];
+        at += c.bytes / sizeof(double);
+    }
+    return cudaSuccess;
+}
+
 cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies)
 {
     cudaError_t e = staging_ensure(ctx);
@@ -239,6 +304,7 @@ cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& co
     struct Part {
         char* dst;
         size_t off, bytes;
+        bool add;
     };
     std::vector<std::vector<Part>> pending(kStageChunks);
     int slot = 0;
@@ -248,8 +314,11 @@ cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& co
         if (r != cudaSuccess) return r;
         const char* base = ctx->stage + (size_t)k * kStageChunk;
         std::vector<Segment> segs;
-        for (const Part& p : pending[k]) segs.push_back(Segment{p.dst, base + p.off, p.bytes});
+        for (const Part& p : pending[k])
+            if (!p.add) segs.push_back(Segment{p.dst, base + p.off, p.bytes});
         copy_segments(ctx, segs);
+        for (const Part& p : pending[k])
+            if (p.add) add_doubles(ctx, reinterpret_cast<double*>(p.dst), reinterpret_cast<const double*>(base + p.off), p.bytes / sizeof(double));
         pending[k].clear();
         return cudaSuccess;
     };
@@ -267,6 +336,7 @@ cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& co
         char* dst = static_cast<char*>(c.dst_host);
         const char* src = static_cast<const char*>(c.src_dev);
         size_t bytes = c.bytes;
+        used = std::min((used + 15) & ~size_t(15), kStageChunk);   // doubles are read in place
         while (bytes > 0 && e == cudaSuccess) {
             if (used == kStageChunk) {
                 e = advance();
@@ -274,7 +344,7 @@ cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& co
             }
             const size_t k = std::min(bytes, kStageChunk - used);
             e = cudaMemcpyAsync(ctx->stage + (size_t)slot * kStageChunk + used, src, k, cudaMemcpyDeviceToHost, s);
-            pending[slot].push_back(Part{dst, used, k});
+            pending[slot].push_back(Part{dst, used, k, c.add});
             used += k;
             dst += k;
             src += k;
