@@ -284,6 +284,7 @@ cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>
         const cudaError_t e = cudaMemcpyAsync(dst, c.src_dev, c.bytes, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return e;
     }
+    if (added == 0) return cudaSuccess;
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
     at = 0;

@@ -90,7 +90,8 @@ struct InCopy {
 };
 cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies);
 
-// copy_out for a call's results: plain copies and one wait below kRingBytes in all.
+// copy_out for a call's results: plain copies below kRingBytes in all, complete once the
+// caller has synchronised `s`.
 cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies);
 
 }  // namespace fm
