@@ -216,6 +216,13 @@ struct SceneBuild {
         pieces.push_back(Piece{host, sizeof(T) * count, block_bytes, static_cast<void*>(field)});
         block_bytes += sizeof(T) * count;
     }
+
+    // Whether the BVH build reads a piece.
+    bool is_geometry(const Piece& p) const
+    {
+        const DevScene& S = sc->dev;
+        return p.field == &S.tri_pos || p.field == &S.rects || p.field == &S.spheres;
+    }
 };
 
 // Validates a description and prepares everything host-side: derived arrays, lights and
@@ -639,63 +646,40 @@ fm_status create_scenes(fm_ctx* ctx, int32_t n, const fm_scene_desc* const* desc
     auto fail_cuda = [&](cudaError_t e, const char* where) {
         return fail(FM_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
     };
-    size_t next_group = 0;
-    for (int32_t i = 0; i < n; ++i) {
-        SceneBuild& B = builds[i];
-        fm_scene* sc = B.sc;
-        DevScene& S = sc->dev;
-        cudaStream_t bs = ctx->build_streams[(size_t)i % ctx->build_streams.size()];
-        cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&B.d_block), B.block_bytes, cs);
-        if (e != cudaSuccess) return fail_cuda(e, "scene allocation");
-        sc->allocations.push_back(B.d_block);
-        sc->d_dev = reinterpret_cast<DevScene*>(B.d_block);
-        if (B.rgb_bytes) {
-            e = cudaMallocAsync(reinterpret_cast<void**>(&B.d_rgb), B.rgb_bytes, cs);
+    // A group's geometry crosses first, for all its scenes, and its BVH build starts behind it
+    // while textures and shading data follow: the build needs only the geometry, and waiting
+    // for the whole upload left the GPU idle for most of it.
+    auto padding = [](size_t end, size_t off) { return off - end < kAlign ? off - end : 0; };
+    const size_t nstreams = ctx->build_streams.size();
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+        Group& g = groups[gi];
+        // builds have the last two streams to themselves
+        cudaStream_t gs = ctx->build_streams[nstreams - 1 - gi % 2];
+        for (int32_t i = g.first; i < g.first + g.count; ++i) {
+            SceneBuild& B = builds[i];
+            fm_scene* sc = B.sc;
+            cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&B.d_block), B.block_bytes, cs);
             if (e != cudaSuccess) return fail_cuda(e, "scene allocation");
-        }
-        for (const Piece& p : B.pieces) {
-            const void* dp = B.d_block + p.off;
-            std::memcpy(p.field, &dp, sizeof(dp));
-        }
-        for (size_t t = 0; t < B.tex_pieces.size(); ++t)
-            sc->textures[t].texels = reinterpret_cast<const float4*>(B.d_block + B.tex_pieces[t].off);
-        // pieces of a block (and of the RGB staging) that only alignment padding separates
-        // go to the device as one copy; the float4 texel regions in between are not copied
-        auto padding = [](size_t end, size_t off) { return off - end < kAlign ? off - end : 0; };
-        size_t end = sizeof(DevScene);
-        for (const Piece& p : B.pieces) {
-            stager.put(B.d_block + p.off, p.src, p.bytes, padding(end, p.off));
-            end = p.off + p.bytes;
-        }
-        end = 0;
-        for (const TexPiece& t : B.tex_pieces) {
-            stager.put(B.d_rgb + t.rgb_off, t.src, t.texels * 3 * sizeof(float), padding(end, t.rgb_off));
-            end = t.rgb_off + t.texels * 3 * sizeof(float);
+            sc->allocations.push_back(B.d_block);
+            sc->d_dev = reinterpret_cast<DevScene*>(B.d_block);
+            if (B.rgb_bytes) {
+                e = cudaMallocAsync(reinterpret_cast<void**>(&B.d_rgb), B.rgb_bytes, cs);
+                if (e != cudaSuccess) return fail_cuda(e, "scene allocation");
+            }
+            for (const Piece& p : B.pieces) {
+                const void* dp = B.d_block + p.off;
+                std::memcpy(p.field, &dp, sizeof(dp));
+                if (B.is_geometry(p)) stager.put(B.d_block + p.off, p.src, p.bytes);
+            }
+            for (size_t t = 0; t < B.tex_pieces.size(); ++t)
+                sc->textures[t].texels = reinterpret_cast<const float4*>(B.d_block + B.tex_pieces[t].off);
         }
         stager.flush();
         if (stager.err != cudaSuccess) return fail_cuda(stager.err, "scene upload");
-        // the scene's device work follows its copies, on its builder stream
-        e = cudaEventRecord(ctx->build_events[0], cs);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(bs, ctx->build_events[0], 0);
-        if (e != cudaSuccess) return fail_cuda(e, "scene upload");
-        for (const TexPiece& t : B.tex_pieces)
-            launch_rgb_to_texels(bs, reinterpret_cast<const float*>(B.d_rgb + t.rgb_off),
-                                 reinterpret_cast<float4*>(B.d_block + t.off), t.texels, ctx->num_sms);
-        if (B.d_rgb) {
-            cudaFreeAsync(B.d_rgb, bs);
-            B.d_rgb = nullptr;
-        }
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return fail_cuda(e, "texel expansion");
-        if (B.env_light_desc >= 0) {
-            st = env_build_tables(ctx, bs, sc, sc->textures[S.env.tex], S.env);
-            if (st != FM_OK) return fail(st, ctx->error);
-        }
-        // the group's last scene is on the device: build the group's BVHs on a builder
-        // stream while the next groups upload
-        Group& g = groups[next_group];
-        if (i == g.first + g.count - 1) {
-            ++next_group;
+        {
+            cudaError_t e = cudaEventRecord(ctx->build_events[0], cs);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(gs, ctx->build_events[0], 0);
+            if (e != cudaSuccess) return fail_cuda(e, "scene build");
             std::vector<PrimSource> srcs((size_t)g.count);
             for (int k = 0; k < g.count; ++k) {
                 const DevScene& D = builds[(size_t)(g.first + k)].sc->dev;
@@ -707,13 +691,65 @@ fm_status create_scenes(fm_ctx* ctx, int32_t n, const fm_scene_desc* const* desc
                 p.rects = D.rects;
                 p.spheres = D.spheres;
             }
-            cudaStream_t gs = ctx->build_streams[(next_group - 1) % ctx->build_streams.size()];
-            e = cudaStreamWaitEvent(gs, ctx->build_events[0], 0);
-            if (e != cudaSuccess) return fail_cuda(e, "scene build");
             std::string err;
             if (bvh_build_batch_begin(gs, ctx->capture_stream, srcs.data(), g.count, g.h_pinned, ctx->num_sms, g.job,
                                       g.bvh, err) != 0)
                 return fail(FM_ERR_CUDA, err);
+        }
+        for (int32_t i = g.first; i < g.first + g.count; ++i) {
+            SceneBuild& B = builds[i];
+            fm_scene* sc = B.sc;
+            DevScene& S = sc->dev;
+            cudaStream_t bs = ctx->build_streams[(size_t)i % (nstreams - 2)];
+            // textures first, as the environment's tables are built from one.  Pieces of the
+            // RGB staging (and of a block) that only alignment padding separates go to the
+            // device as one copy; the float4 texel regions in between are not copied.
+            size_t end = 0;
+            for (const TexPiece& t : B.tex_pieces) {
+                stager.put(B.d_rgb + t.rgb_off, t.src, t.texels * 3 * sizeof(float), padding(end, t.rgb_off));
+                end = t.rgb_off + t.texels * 3 * sizeof(float);
+            }
+            auto put_rest = [&]() {
+                size_t at = sizeof(DevScene);
+                bool adjacent = true;   // nothing already on the device lies between `at` and the piece
+                for (const Piece& p : B.pieces) {
+                    if (B.is_geometry(p)) {
+                        adjacent = false;
+                    } else {
+                        stager.put(B.d_block + p.off, p.src, p.bytes, adjacent ? padding(at, p.off) : 0);
+                        adjacent = true;
+                    }
+                    at = p.off + p.bytes;
+                }
+                stager.flush();
+            };
+            // a large scene's tables are built while its shading data crosses; a small one's
+            // copies go together
+            const bool split = B.block_bytes > kStageChunk * kStageChunks;
+            if (split)
+                stager.flush();
+            else
+                put_rest();
+            if (stager.err != cudaSuccess) return fail_cuda(stager.err, "scene upload");
+            // the scene's device work follows its copies, on its builder stream
+            cudaError_t e = cudaEventRecord(ctx->build_events[0], cs);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(bs, ctx->build_events[0], 0);
+            if (e != cudaSuccess) return fail_cuda(e, "scene upload");
+            for (const TexPiece& t : B.tex_pieces)
+                launch_rgb_to_texels(bs, reinterpret_cast<const float*>(B.d_rgb + t.rgb_off),
+                                     reinterpret_cast<float4*>(B.d_block + t.off), t.texels, ctx->num_sms);
+            if (B.d_rgb) {
+                cudaFreeAsync(B.d_rgb, bs);
+                B.d_rgb = nullptr;
+            }
+            e = cudaGetLastError();
+            if (e != cudaSuccess) return fail_cuda(e, "texel expansion");
+            if (B.env_light_desc >= 0) {
+                st = env_build_tables(ctx, bs, sc, sc->textures[S.env.tex], S.env);
+                if (st != FM_OK) return fail(st, ctx->error);
+            }
+            if (split) put_rest();
+            if (stager.err != cudaSuccess) return fail_cuda(stager.err, "scene upload");
         }
     }
     // wait for the builds; then every scene's record
