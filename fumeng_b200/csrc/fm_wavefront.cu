@@ -41,14 +41,15 @@ namespace fm {
 
 namespace {
 
-constexpr int kNeedItem = -2;
-constexpr int kDone = -1;
 // slot flags (depth in bits 8..): a continuation ray was queued / shadow or MIS rays of
 // this slot are queued, both set by the shading kernels and read by the logic kernel
 constexpr int kNextCont = 1;
 constexpr int kPending = 2;
 // adjoint renders: the slot is replaying its sample's path (second pass)
 constexpr int kReplay = 4;
+// the slot has no work item yet / will get none any more
+constexpr int kNeedItem = 8;
+constexpr int kDone = 16;
 // queue counters: two sets of the three ray queues (the one being filled for the next trace
 // and the one being traced; they change places every iteration, see WfState::qw), slots
 // still holding work, the shading queues (two classes, and in adjoint renders two more
@@ -77,10 +78,10 @@ struct WfState {
     int64_t total_items;
     unsigned long long* next_item;
     // per slot
-    int64_t* item;        // global work item, or kNeedItem / kDone
+    int64_t* item;        // global work item (unless kNeedItem or kDone)
     int32_t* k;           // sample within the item
     int32_t* view;
-    int32_t* flags;       // kNextCont | kPending | depth << 8
+    int32_t* flags;       // kNextCont | kPending | kReplay | kNeedItem | kDone | depth << 8
     uint64_t* rng;
     float4* beta;
     float4* col;
@@ -1089,140 +1090,194 @@ __global__ void __launch_bounds__(256) k_wf_shade_replay(WfState st)
 
 // Per slot, after the shading kernels: a sample with neither a continuation ray nor
 // rays in flight is finished: its colour (with the shadow, MIS and emission
-// contributions the resolve kernel added; adjoint renders fold this iteration's in from
+// contributions the resolve kernels added; adjoint renders fold this iteration's in from
 // acc first) goes into the item's Kahan sum and the slot starts its next sample, or
 // takes a new work item.
-// Six blocks per SM (40 registers, 12 B of spills): the slot loop waits on dependent
-// loads, and the extra resident warps beat the uncapped 54 registers (299.8 against
-// 301.9 ms per batched step; eight blocks, 32 registers: 303.0 ms).
-template <bool ADJ>
-__global__ void __launch_bounds__(256, 6) k_wf_logic(WfState st)
+// Most slots of most iterations have rays in flight or no work left, so a block first
+// looks at the flags of PER slots per thread (16 bytes at once for four) and lists the slots
+// that need more; the long part then runs with full warps over the list.  Deciding slot
+// by slot ran it at 18-20 lanes of 32 and had every slot pass the block-wide queue append:
+// all kernels but the trace kernel took 30.5 -> 28.9 ms of the 16-scene batch and 0.93 ->
+// 0.74 ms of the Cornell box.  Adjoint renders keep one slot per thread (PER = 1): they fold
+// acc into col for every slot with rays in flight, 16-byte records that must be read in
+// lane order (four per thread: 11.3 -> 13.6 ms for 4 views).
+// Five blocks per SM (48 registers): the long part waits on dependent loads; four and six
+// are within 1 %.
+template <bool ADJ, int PER>
+__global__ void __launch_bounds__(256, 5) k_wf_logic(WfState st)
 {
     unsigned long long n_paths = 0, n_nans = 0;
     unsigned n_active = 0;
     __shared__ unsigned s_app[2];
+    __shared__ unsigned s_n;
+    __shared__ uint16_t s_list[256 * PER];
     const int cont_qc = kQcCont;
-    for (int64_t s0 = blockIdx.x * (int64_t)blockDim.x; s0 < st.pool; s0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t s64 = s0 + threadIdx.x;
-        const int slot = (int)s64;
-        const bool in_range = s64 < st.pool;
-        int64_t item = in_range ? st.item[slot] : (int64_t)kDone;
-        bool need_new = item == kNeedItem;
-        bool enqueue_cont = false;
-        bool alive = false;
-        // the sample to start (one start_sample call for every case below, so that the
-        // lanes of a warp generate their camera rays together)
-        int s_vid = 0, s_k = 0, s_flags = 0;
-        int64_t s_local = 0;
-        if (item >= 0) {
-            const int flags = st.flags[slot];
-            const bool cont = (flags & (kNextCont | kPending)) != 0;
-            // the sample's radiance so far: forward renders add contributions to col
-            // directly, adjoint renders collect this iteration's in acc (the replay needs
-            // the radiance before them), added to col here
-            f3 col = mk(0.0f);
-            if (ADJ) {
-                const float4 a4 = st.acc[slot];
-                const float4 c4 = st.col[slot];
-                col = f3{c4.x + a4.x, c4.y + a4.y, c4.z + a4.z};
-                if (a4.x != 0.0f || a4.y != 0.0f || a4.z != 0.0f) st.acc[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            } else if (!cont) {
-                const float4 c4 = st.col[slot];
-                col = f3{c4.x, c4.y, c4.z};
-            }
-            if (cont) {
-                if (ADJ) st.col[slot] = make_float4(col.x, col.y, col.z, 0.0f);
-                st.flags[slot] = flags & ~(kNextCont | kPending);
-                alive = true;
-            } else if (ADJ && !(flags & kReplay)) {
-                // primal pass of this sample done: keep L, add it to the image, replay
-                const int vid = st.view[slot];
-                const WfView& V = st.views[vid];
-                st.lp[slot] = make_float4(col.x, col.y, col.z, 0.0f);
-                s_k = st.k[slot];
-                float4 sum, cmp;
-                item_sums(st, slot, s_k, sum, cmp);
-                kahan_add4(sum, cmp, col);
-                st.isum[slot] = sum;
-                st.icomp[slot] = cmp;
-                s_vid = vid;
-                s_local = item - V.item_base;
-                s_flags = kReplay;
-                enqueue_cont = true;
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = blockIdx.x * (int64_t)(256 * PER); base < st.pool; base += (int64_t)gridDim.x * (256 * PER)) {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        {
+            const int64_t first = base + PER * (int)threadIdx.x;
+            const bool whole = first + PER <= st.pool;
+            int f[PER];
+            if (PER == 4 && whole) {
+                const int4 f4 = *reinterpret_cast<const int4*>(st.flags + first);
+                f[0] = f4.x;
+                f[PER > 1 ? 1 : 0] = f4.y;
+                f[PER > 2 ? 2 : 0] = f4.z;
+                f[PER > 3 ? 3 : 0] = f4.w;
             } else {
-                const int vid = st.view[slot];
-                const WfView& V = st.views[vid];
-                if (ADJ) {
-                    // the last vertex's record (its NEE / MIS rays are resolved)
-                    const float4 l4 = st.lp[slot];
-                    const f3 R = f3{l4.x - col.x, l4.y - col.y, l4.z - col.z};
-                    flush_vertex(st, vid, slot, pixel_delta(st, slot, V) * R);
-                }
-                ++n_paths;
-                if (!isfinite(col.x) || !isfinite(col.y) || !isfinite(col.z)) ++n_nans;
-                const int k = st.k[slot];
-                float4 sum, cmp;
-                // the primal pass has added an adjoint render's sample already
-                item_sums(st, slot, ADJ ? k + 1 : k, sum, cmp);
-                if (!ADJ) kahan_add4(sum, cmp, clamp_sample(V.cfg, col));
-                const int kdone = k + 1;
-                const int64_t local = item - V.item_base;
-                const int npix = V.cfg.width * V.cfg.height;
-                const int chunk_index = (int)(local / npix);
-                if (kdone >= item_samples(V, chunk_index)) {
-                    float4* P = V.partial + V.partial_f4 * (size_t)local;
-                    P[0] = sum;
-                    if (st.aov) {
-                        P[1] = st.asum[slot];
-                        P[2] = st.nsum[slot];
+                for (int k = 0; k < PER; ++k) f[k] = first + k < st.pool ? st.flags[first + k] : kDone;
+            }
+            unsigned todo = 0;
+#pragma unroll
+            for (int k = 0; k < PER; ++k) {
+                if (f[k] & kDone) continue;
+                if (!(f[k] & kNeedItem) && (f[k] & (kNextCont | kPending))) {
+                    ++n_active;
+                    f[k] &= ~(kNextCont | kPending);
+                    st.flags[first + k] = f[k];
+                    if (ADJ) {
+                        const float4 a4 = st.acc[first + k];
+                        if (a4.x != 0.0f || a4.y != 0.0f || a4.z != 0.0f) {
+                            const float4 c4 = st.col[first + k];
+                            st.col[first + k] = make_float4(c4.x + a4.x, c4.y + a4.y, c4.z + a4.z, 0.0f);
+                            st.acc[first + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        }
                     }
-                    need_new = true;
                 } else {
+                    todo |= 1u << k;
+                }
+            }
+            const int mine = __popc(todo);
+            int upto = mine;
+            for (int off = 1; off < 32; off <<= 1) {
+                const int o = __shfl_up_sync(0xffffffffu, upto, off);
+                if (lane >= off) upto += o;
+            }
+            unsigned at = 0;
+            if (lane == 31 && upto) at = atomicAdd(&s_n, (unsigned)upto);
+            at = __shfl_sync(0xffffffffu, at, 31) + (unsigned)(upto - mine);
+#pragma unroll
+            for (int k = 0; k < PER; ++k)
+                if ((todo >> k) & 1u) s_list[at++] = (uint16_t)(PER * threadIdx.x + k);
+        }
+        __syncthreads();
+        const int n = (int)s_n;
+        for (int j0 = 0; j0 < n; j0 += 256) {
+            const int j = j0 + (int)threadIdx.x;
+            const bool listed = j < n;
+            const int slot = listed ? (int)(base + s_list[j]) : 0;
+            const int flags = listed ? st.flags[slot] : kDone;
+            bool need_new = (flags & kNeedItem) != 0;
+            bool enqueue_cont = false;
+            // the sample to start (one start_sample call for every case below, so that the
+            // lanes of a warp generate their camera rays together)
+            int s_vid = 0, s_k = 0, s_flags = 0;
+            int64_t s_local = 0;
+            if (listed && !need_new) {
+                const int64_t item = st.item[slot];
+                // the sample's radiance: forward renders add contributions to col directly,
+                // adjoint renders collect this iteration's in acc (the replay needs the radiance
+                // before them)
+                const float4 c4 = st.col[slot];
+                f3 col = f3{c4.x, c4.y, c4.z};
+                if (ADJ) {
+                    const float4 a4 = st.acc[slot];
+                    col = f3{c4.x + a4.x, c4.y + a4.y, c4.z + a4.z};
+                    if (a4.x != 0.0f || a4.y != 0.0f || a4.z != 0.0f) st.acc[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+                if (ADJ && !(flags & kReplay)) {
+                    // primal pass of this sample done: keep L, add it to the image, replay
+                    const int vid = st.view[slot];
+                    const WfView& V = st.views[vid];
+                    st.lp[slot] = make_float4(col.x, col.y, col.z, 0.0f);
+                    s_k = st.k[slot];
+                    float4 sum, cmp;
+                    item_sums(st, slot, s_k, sum, cmp);
+                    kahan_add4(sum, cmp, col);
                     st.isum[slot] = sum;
                     st.icomp[slot] = cmp;
-                    st.k[slot] = kdone;
                     s_vid = vid;
-                    s_local = local;
-                    s_k = kdone;
+                    s_local = item - V.item_base;
+                    s_flags = kReplay;
                     enqueue_cont = true;
-                }
-            }
-        }
-        // new work items for slots that finished theirs (one atomic per warp)
-        {
-            const unsigned mask = __activemask();
-            const unsigned b = __ballot_sync(mask, need_new);
-            if (need_new) {
-                const int leader = __ffs(b) - 1;
-                unsigned long long base = 0;
-                if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(st.next_item, (unsigned long long)__popc(b));
-                base = __shfl_sync(b, base, leader);
-                const int64_t it = (int64_t)(base + __popc(b & lanemask_lt()));
-                if (it >= st.total_items) {
-                    st.item[slot] = kDone;
                 } else {
-                    const int vid = find_view(st, it);
+                    const int vid = st.view[slot];
                     const WfView& V = st.views[vid];
-                    st.item[slot] = it;
-                    st.view[slot] = vid;
-                    st.k[slot] = 0;
-                    if (st.aov) st.asum[slot] = st.nsum[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    s_vid = vid;
-                    s_local = it - V.item_base;
-                    s_k = 0;
-                    enqueue_cont = true;
+                    if (ADJ) {
+                        // the last vertex's record (its NEE / MIS rays are resolved)
+                        const float4 l4 = st.lp[slot];
+                        const f3 R = f3{l4.x - col.x, l4.y - col.y, l4.z - col.z};
+                        flush_vertex(st, vid, slot, pixel_delta(st, slot, V) * R);
+                    }
+                    ++n_paths;
+                    if (!isfinite(col.x) || !isfinite(col.y) || !isfinite(col.z)) ++n_nans;
+                    const int k = st.k[slot];
+                    float4 sum, cmp;
+                    // the primal pass has added an adjoint render's sample already
+                    item_sums(st, slot, ADJ ? k + 1 : k, sum, cmp);
+                    if (!ADJ) kahan_add4(sum, cmp, clamp_sample(V.cfg, col));
+                    const int kdone = k + 1;
+                    const int64_t local = item - V.item_base;
+                    const int npix = V.cfg.width * V.cfg.height;
+                    const int chunk_index = (int)(local / npix);
+                    if (kdone >= item_samples(V, chunk_index)) {
+                        float4* P = V.partial + V.partial_f4 * (size_t)local;
+                        P[0] = sum;
+                        if (st.aov) {
+                            P[1] = st.asum[slot];
+                            P[2] = st.nsum[slot];
+                        }
+                        need_new = true;
+                    } else {
+                        st.isum[slot] = sum;
+                        st.icomp[slot] = cmp;
+                        st.k[slot] = kdone;
+                        s_vid = vid;
+                        s_local = local;
+                        s_k = kdone;
+                        enqueue_cont = true;
+                    }
                 }
             }
+            // new work items for slots that finished theirs (one atomic per warp)
+            {
+                const unsigned mask = __activemask();
+                const unsigned b = __ballot_sync(mask, need_new);
+                if (need_new) {
+                    const int leader = __ffs(b) - 1;
+                    unsigned long long base = 0;
+                    if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(st.next_item, (unsigned long long)__popc(b));
+                    base = __shfl_sync(b, base, leader);
+                    const int64_t it = (int64_t)(base + __popc(b & lanemask_lt()));
+                    if (it >= st.total_items) {
+                        st.flags[slot] = kDone;
+                    } else {
+                        const int vid = find_view(st, it);
+                        const WfView& V = st.views[vid];
+                        st.item[slot] = it;
+                        st.view[slot] = vid;
+                        st.k[slot] = 0;
+                        if (st.aov) st.asum[slot] = st.nsum[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        s_vid = vid;
+                        s_local = it - V.item_base;
+                        s_k = 0;
+                        enqueue_cont = true;
+                    }
+                }
+            }
+            if (enqueue_cont) start_sample(st, slot, st.views[s_vid], s_local, s_k, s_flags);
+            const int64_t q = block_append<1>(st.qw, &cont_qc, enqueue_cont ? 0 : -1, s_app);
+            if (enqueue_cont) {
+                if (q < st.cap_cont)
+                    st.cont_q[q] = slot;
+                else
+                    atomicOr(st.status, 2u);
+            }
+            if (enqueue_cont) ++n_active;
         }
-        if (enqueue_cont) start_sample(st, slot, st.views[s_vid], s_local, s_k, s_flags);
-        const int64_t q = block_append<1>(st.qw, &cont_qc, enqueue_cont ? 0 : -1, s_app);
-        if (enqueue_cont) {
-            if (q < st.cap_cont)
-                st.cont_q[q] = slot;
-            else
-                atomicOr(st.status, 2u);
-        }
-        if (enqueue_cont || alive) ++n_active;
+        __syncthreads();   // the list is free again
     }
     for (int off = 16; off > 0; off >>= 1) {
         n_paths += __shfl_xor_sync(0xffffffffu, n_paths, off);
@@ -1256,8 +1311,7 @@ __global__ void k_wf_init(WfState st)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) st.tspan[0] = ~0ull;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < st.pool; s += (int64_t)gridDim.x * blockDim.x) {
-        st.item[s] = kNeedItem;
-        st.flags[s] = 0;
+        st.flags[s] = kNeedItem;
         st.acc[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         st.col[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
@@ -1599,7 +1653,9 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     const int trace_grid = sms * (1024 / tune.trace_block);
     const size_t trace_smem = kTraceSmemPerThread * (size_t)tune.trace_block;
     const int shade_grid = (int)std::min<int64_t>((pool + tune.shade_block - 1) / tune.shade_block, (int64_t)sms * 32);
-    const int logic_grid = (int)std::min<int64_t>((pool + 255) / 256, (int64_t)sms * 32);
+    // slots per thread of the logic kernel: four where that still leaves several blocks per SM
+    const bool logic4 = !ADJ && pool >= (int64_t)sms * 4096;
+    const int logic_grid = (int)std::min<int64_t>((pool + 255) / (logic4 ? 1024 : 256), (int64_t)sms * 32);
     const int resolve_grid = sms * 16;
     // Bound on iterations: every sample takes at most depth + 1 iterations and a slot
     // runs its samples one after another.
@@ -1653,7 +1709,10 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
             }
             after(c->join[1], s2, s);
             after(c->join[0], s1, s);
-            k_wf_logic<ADJ><<<logic_grid, 256, 0, s>>>(x);
+            if (logic4)
+                k_wf_logic<false, 4><<<logic_grid, 256, 0, s>>>(x);
+            else
+                k_wf_logic<ADJ, 1><<<logic_grid, 256, 0, s>>>(x);
             if (ADJ) k_wf_grad_scatter<<<sms * 8, 256, 0, s>>>(x);
             if (tune.profile) cudaEventRecordWithFlags(pev[3 * it + 2], s, cudaEventRecordExternal);
         }
