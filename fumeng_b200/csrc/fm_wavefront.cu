@@ -1072,12 +1072,14 @@ FM_D void shade_vertices(const WfState& st)
     if ((threadIdx.x & 31) == 0 && n_bounces) atomicAdd(&st.cnt->bounces, n_bounces);
 }
 
-// The shading kernels.  Forward ones are capped at 80 registers (three 256-thread blocks
-// per SM): the extra occupancy outweighs the spills of the Disney kernel.  The replay
-// kernels of adjoint renders keep the compiler's allocation (their dual-number code
-// spills heavily under a cap).
+// The shading kernels.  The forward Disney kernel is capped at 64 registers (four 256-thread
+// blocks per SM): it waits on dependent loads and instruction fetch, and the extra warps
+// outweigh its spills (16-scene batch, all kernels but trace: 31.5 / 30.5 / 29.9 ms with two /
+// three / four blocks).  The other materials' kernel keeps 80 (two / three / four / five
+// blocks: 32.4 / 30.5 / 30.6 / 31.0 ms).  The replay kernels of adjoint renders keep the
+// compiler's allocation (their dual-number code spills heavily under a cap).
 template <int CLS>
-__global__ void __launch_bounds__(256, 3) k_wf_shade(WfState st)
+__global__ void __launch_bounds__(256, CLS == kClsDisney ? 4 : 3) k_wf_shade(WfState st)
 {
     shade_vertices<CLS, false>(st);
 }
