@@ -1111,9 +1111,7 @@ __global__ void __launch_bounds__(256) k_wf_shade_replay(WfState st)
 // that need more; the long part then runs with full warps over the list.  Deciding slot
 // by slot ran it at 18-20 lanes of 32 and had every slot pass the block-wide queue append:
 // all kernels but the trace kernel took 30.5 -> 28.9 ms of the 16-scene batch and 0.93 ->
-// 0.74 ms of the Cornell box.  Adjoint renders keep one slot per thread (PER = 1): they fold
-// acc into col for every slot with rays in flight, 16-byte records that must be read in
-// lane order (four per thread: 11.3 -> 13.6 ms for 4 views).
+// 0.74 ms of the Cornell box; in an adjoint render of 4 views 10.55 -> 10.47 ms.
 // Five blocks per SM (48 registers): the long part waits on dependent loads; four and six
 // are within 1 %.
 template <bool ADJ, int PER>
@@ -1667,7 +1665,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     const size_t trace_smem = kTraceSmemPerThread * (size_t)tune.trace_block;
     const int shade_grid = (int)std::min<int64_t>((pool + tune.shade_block - 1) / tune.shade_block, (int64_t)sms * 32);
     // slots per thread of the logic kernel: four where that still leaves several blocks per SM
-    const bool logic4 = !ADJ && pool >= (int64_t)sms * 4096;
+    const bool logic4 = pool >= (int64_t)sms * 4096;
     const int logic_grid = (int)std::min<int64_t>((pool + 255) / (logic4 ? 1024 : 256), (int64_t)sms * 32);
     const int resolve_grid = sms * 16;
     // Bound on iterations: every sample takes at most depth + 1 iterations and a slot
@@ -1723,7 +1721,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
             after(c->join[1], s2, s);
             after(c->join[0], s1, s);
             if (logic4)
-                k_wf_logic<false, 4><<<logic_grid, 256, 0, s>>>(x);
+                k_wf_logic<ADJ, 4><<<logic_grid, 256, 0, s>>>(x);
             else
                 k_wf_logic<ADJ, 1><<<logic_grid, 256, 0, s>>>(x);
             if (ADJ) k_wf_grad_scatter<<<sms * 8, 256, 0, s>>>(x);
