@@ -217,7 +217,8 @@ typedef struct {
  * holder used by every other call.  A context keeps its wavefront workspace between
  * renders (path-state and queue buffers sized to the largest pool and queues seen: for
  * forward renders about 332 B plus 100 B per light per path slot, 2.2 GB at 2^22 slots
- * and two lights, of which 48 B plus 48 B per light are left out when memory is short; more for adjoint renders; pinned staging; the instantiated render
+ * and two lights, of which 48 B plus 48 B per light are left out when memory is short;
+ * fm_render uses 2^21 slots, up to 2^23 for renders of 1.5 samples per slot and more; more for adjoint renders; pinned staging; the instantiated render
  * graph) and releases it in fm_ctx_destroy. */
 fm_status fm_ctx_create(int device, fm_ctx** out);
 void fm_ctx_destroy(fm_ctx* ctx);
