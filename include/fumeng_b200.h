@@ -218,8 +218,9 @@ typedef struct {
  * renders (path-state and queue buffers sized to the largest pool and queues seen: for
  * forward renders about 332 B plus 100 B per light per path slot, 2.2 GB at 2^22 slots
  * and two lights, of which 48 B plus 48 B per light are left out when memory is short;
- * fm_render uses 2^21 slots, up to 2^23 for renders of 1.5 samples per slot and more; more for adjoint renders; pinned staging; the instantiated render
- * graph) and releases it in fm_ctx_destroy. */
+ * more for adjoint renders; pinned staging; the instantiated render graph) and releases it
+ * in fm_ctx_destroy.  fm_render uses 2^21 slots, or up to 2^23 where a render has 1.5
+ * samples or more per slot and the workspace stays below 8 GB. */
 fm_status fm_ctx_create(int device, fm_ctx** out);
 void fm_ctx_destroy(fm_ctx* ctx);
 const char* fm_last_error(const fm_ctx* ctx);
