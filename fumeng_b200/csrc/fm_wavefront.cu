@@ -931,7 +931,8 @@ FM_D void shade_vertices(const WfState& st)
                     J.env = L.kind == LK_ENV;
                 }
             };
-            auto mis_job = [&](const BsdfSample& ms, ShadeJob& J) {
+            auto mis_job = [&](ShadeJob& J) {
+                const BsdfSample ms = bsdf_sample<CLS>(b, h.wo, rng_3d(rng));
                 const bool ok = length(ms.f) >= kEpsPdf && ms.pdf >= kEpsPdf;
                 const int64_t q = ADJ ? wagg_append_grouped(&st.qw[kQcMis], ok) : wagg_append(&st.qw[kQcMis], ok);
                 if (!ok) return;
@@ -955,7 +956,8 @@ FM_D void shade_vertices(const WfState& st)
                     J.sdelta = ms.delta;
                 }
             };
-            auto cont_job = [&](const BsdfSample& sc, ShadeJob& J) {
+            auto cont_job = [&](ShadeJob& J) {
+                const BsdfSample sc = bsdf_sample<CLS>(b, h.wo, rng_3d(rng));
                 if (!(length(sc.f) >= kEpsPdf && sc.pdf >= kEpsPdf)) return;
                 beta *= sc.f * absdot(h.ng, sc.wi) / sc.pdf;
                 if (depth >= V.cfg.depth) return;
@@ -979,15 +981,12 @@ FM_D void shade_vertices(const WfState& st)
                 for (int j = 0; j < njobs; ++j) {
                     const int r = j == njobs - 1 ? -1 : j % (nl + 1);
                     ShadeJob J;
-                    if (r >= 0 && r < nl) {
+                    if (r < 0)
+                        cont_job(J);
+                    else if (r == nl)
+                        mis_job(J);
+                    else
                         nee_job(r, J);
-                    } else {
-                        const BsdfSample bs = bsdf_sample<CLS>(b, h.wo, rng_3d(rng));
-                        if (r < 0)
-                            cont_job(bs, J);
-                        else
-                            mis_job(bs, J);
-                    }
                     if (J.kind == 0) continue;
                     BsdfGrads bg;
                     const bool grads = tgt >= 0 && !(J.kind == 2 && J.sdelta && CLS == kClsSimple);
@@ -1051,22 +1050,12 @@ FM_D void shade_vertices(const WfState& st)
                     }
                 }
             } else {
-                // one copy of the BSDF sampling code for the MIS sample and the continuation:
-                // the Disney kernel waits on instruction fetch (against two copies: 1.3 M
-                // triangles at 1080p, kernels but trace 2.32 -> 2.15 ms, replay kernels
-                // likewise, adjoint of 4 views 10.9 -> 10.55 ms)
                 ShadeJob J;
-#pragma unroll 1
-                for (int kk = 0; kk <= V.cfg.direct_loop; ++kk) {
-                    const bool last = kk == V.cfg.direct_loop;
-                    if (!last)
-                        for (int r = 0; r < nl; ++r) nee_job(r, J);
-                    const BsdfSample bs = bsdf_sample<CLS>(b, h.wo, rng_3d(rng));
-                    if (last)
-                        cont_job(bs, J);
-                    else
-                        mis_job(bs, J);
+                for (int kk = 0; kk < V.cfg.direct_loop; ++kk) {
+                    for (int r = 0; r < nl; ++r) nee_job(r, J);
+                    mis_job(J);
                 }
+                cont_job(J);
             }
             st.rng[slot] = rng.state;
             st.flags[slot] = flags;
