@@ -49,7 +49,7 @@ NSCENES = 64
 # DRAM bytes the trace kernel moves per traced ray (read + write, cold L2 at each
 # launch), from an ncu capture of two trace launches of the 8-scene case of this
 # workload (68.8 and 63.1 B per ray); traffic grows with the rays a launch traces.
-TRACE_DRAM_BYTES_PER_RAY = 66.0
+TRACE_DRAM_BYTES_PER_RAY = 64.2
 
 
 def measured_peak_hbm():
