@@ -89,7 +89,7 @@ struct WfState {
     float4* rd;
     float4* hit;
     float4* acc;          // adjoint renders: the iteration's MIS, shadow and emission contributions
-                          // (atomic adds from the resolve kernel; forward renders add them to col)
+                          // (atomic adds from the resolve kernels; forward renders add them to col)
     float4* isum;
     float4* icomp;
     float4* asum;
@@ -123,7 +123,7 @@ struct WfState {
     // adjoint renders only (null otherwise)
     float4* lp;           // primal radiance of the slot's current sample
     float4* dfr;          // [5 per slot] the slot's current vertex: dlw[15] (c*5+i), material, u, v
-    float4* vg;           // [2 per slot] gradient collected for that vertex (g[5]; NEE / MIS, resolve kernel)
+    float4* vg;           // [2 per slot] gradient collected for that vertex (g[5]; NEE / MIS, resolve kernels)
     float4* gq;           // [3 per entry] finished vertices' gradients: g[5], u, v, material, view
     int64_t cap_grad;
     float4* sh_g;         // [3 per shadow ray] g[5], u, v, material, env weight e[3], env score s
