@@ -39,6 +39,12 @@ FM_D f32x2 add2(f32x2 a, f32x2 b)
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+FM_D f32x2 add2_down(f32x2 a, f32x2 b)   // rounded towards minus infinity
+{
+    f32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 FM_D f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
 {
     f32x2 r;
