@@ -30,6 +30,7 @@
 // the launch state (WfState, tuning, iteration bound) is byte-identical.
 #include <cmath>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "fm_bsdf_grad.cuh"
@@ -1363,8 +1364,10 @@ struct WfCache {
     bool adj = false;
     int64_t pool = 0, cap_mis = 0, cap_sh = 0, partial_f4 = 0;
     int32_t nviews = 0;
-    std::vector<void*> allocs;   // state buffers
-    WfState bufs;                // their pointers
+    size_t held = 0;             // device bytes of everything below
+    int64_t builds = 0;          // times the state buffers were allocated
+    std::vector<std::pair<void*, size_t>> allocs;   // state buffers and their bytes
+    WfState bufs;                                   // their pointers
     RayQueue alt;                // forward renders: a second set of ray records (null: none)
     cudaStream_t side[2] = {nullptr, nullptr};   // the branches of an iteration's kernels
     cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr}, fork2 = nullptr;
@@ -1402,13 +1405,57 @@ void wf_cache_drop_graph(WfCache& c)
     c.graph = nullptr;
 }
 
+// Device memory of the workspace; refused beyond the context's limit as the driver refuses
+// it when the device has no more.
+cudaError_t wf_malloc(fm_ctx* ctx, WfCache& c, void** p, size_t bytes)
+{
+    if (ctx->wf_limit > 0 && c.held + bytes > ctx->wf_limit) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e == cudaSuccess) c.held += bytes;
+    return e;
+}
+void wf_free(WfCache& c, cudaStream_t s, void* p, size_t bytes)
+{
+    if (!p) return;
+    cudaFreeAsync(p, s);
+    c.held -= bytes;
+}
+
+// Frees state buffers until `keep` are left.
+void wf_cache_free_allocs(WfCache& c, cudaStream_t s, size_t keep)
+{
+    while (c.allocs.size() > keep) {
+        wf_free(c, s, c.allocs.back().first, c.allocs.back().second);
+        c.allocs.pop_back();
+    }
+}
+
 void wf_cache_free_state(WfCache& c, cudaStream_t s)
 {
-    for (void* p : c.allocs) cudaFreeAsync(p, s);
-    c.allocs.clear();
+    wf_cache_free_allocs(c, s, 0);
     std::memset(&c.bufs, 0, sizeof(c.bufs));
     std::memset(&c.alt, 0, sizeof(c.alt));
     c.pool = c.cap_mis = c.cap_sh = 0;
+}
+
+// Releases a workspace, complete or not.
+void wf_cache_destroy(WfCache*& c, cudaStream_t s)
+{
+    wf_cache_drop_graph(*c);
+    wf_cache_free_state(*c, s);
+    wf_free(*c, s, c->partial, sizeof(float4) * (size_t)c->partial_f4);
+    wf_free(*c, s, c->d_views, sizeof(WfView) * (size_t)c->nviews);
+    wf_free(*c, s, c->cnt, sizeof(Counters));
+    cudaStreamSynchronize(s);
+    if (c->h_views) cudaFreeHost(c->h_views);
+    if (c->h_block) cudaFreeHost(c->h_block);
+    for (cudaStream_t x : c->side)
+        if (x) cudaStreamDestroy(x);
+    for (cudaEvent_t ev : {c->fork, c->fork2, c->join[0], c->join[1], c->e0, c->e1})
+        if (ev) cudaEventDestroy(ev);
+    for (cudaEvent_t ev : c->pev) cudaEventDestroy(ev);
+    delete c;
+    c = nullptr;
 }
 
 // Makes the workspace of `ctx` (forward or adjoint) hold at least the given capacities.
@@ -1427,8 +1474,9 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
             cudaEventCreateWithFlags(&c->fork, nt) != cudaSuccess || cudaEventCreateWithFlags(&c->fork2, nt) != cudaSuccess ||
             cudaEventCreateWithFlags(&c->join[0], nt) != cudaSuccess ||
             cudaEventCreateWithFlags(&c->join[1], nt) != cudaSuccess || cudaEventCreate(&c->e0) != cudaSuccess || cudaEventCreate(&c->e1) != cudaSuccess ||
-            cudaMallocHost(&c->h_block, hb) != cudaSuccess || cudaMallocAsync((void**)&c->cnt, sizeof(Counters), s) != cudaSuccess) {
+            cudaMallocHost(&c->h_block, hb) != cudaSuccess || wf_malloc(ctx, *c, (void**)&c->cnt, sizeof(Counters)) != cudaSuccess) {
             cudaGetLastError();
+            wf_cache_destroy(c, s);
             return set_error(ctx, FM_ERR_OOM, "wavefront: workspace allocation failed");
         }
         char* hp = static_cast<char*>(c->h_block);
@@ -1438,7 +1486,7 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
     }
     if (nviews > c->nviews) {
         wf_cache_drop_graph(*c);
-        if (c->d_views) cudaFreeAsync(c->d_views, s);
+        wf_free(*c, s, c->d_views, sizeof(WfView) * (size_t)c->nviews);
         if (c->h_views) {
             cudaStreamSynchronize(s);
             cudaFreeHost(c->h_views);
@@ -1446,18 +1494,21 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
         c->d_views = nullptr;
         c->h_views = nullptr;
         c->nviews = 0;
-        if (cudaMallocAsync((void**)&c->d_views, sizeof(WfView) * (size_t)nviews, s) != cudaSuccess ||
+        WfView* d = nullptr;
+        if (wf_malloc(ctx, *c, (void**)&d, sizeof(WfView) * (size_t)nviews) != cudaSuccess ||
             cudaMallocHost((void**)&c->h_views, sizeof(WfView) * (size_t)nviews) != cudaSuccess) {
             cudaGetLastError();
+            wf_free(*c, s, d, sizeof(WfView) * (size_t)nviews);
             return set_error(ctx, FM_ERR_OOM, "wavefront: view table allocation failed");
         }
+        c->d_views = d;
         c->nviews = nviews;
     }
     if (partial_f4 > c->partial_f4) {
-        if (c->partial) cudaFreeAsync(c->partial, s);
+        wf_free(*c, s, c->partial, sizeof(float4) * (size_t)c->partial_f4);
         c->partial = nullptr;
         c->partial_f4 = 0;
-        if (cudaMallocAsync((void**)&c->partial, sizeof(float4) * (size_t)partial_f4, s) != cudaSuccess) {
+        if (wf_malloc(ctx, *c, (void**)&c->partial, sizeof(float4) * (size_t)partial_f4) != cudaSuccess) {
             cudaGetLastError();
             return set_error(ctx, FM_ERR_OOM, "wavefront: partial buffer allocation failed");
         }
@@ -1473,8 +1524,9 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
         bool ok = true;
         auto A = [&](auto*& p, size_t count) {
             void* q = nullptr;
-            if (ok && cudaMallocAsync(&q, sizeof(*p) * count, s) == cudaSuccess) {
-                c->allocs.push_back(q);
+            const size_t bytes = sizeof(*p) * count;
+            if (ok && wf_malloc(ctx, *c, &q, bytes) == cudaSuccess) {
+                c->allocs.emplace_back(q, bytes);
                 p = static_cast<std::remove_reference_t<decltype(p)>>(q);
             } else {
                 ok = false;
@@ -1535,16 +1587,14 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
             queue(c->alt);
             if (!ok) {
                 cudaGetLastError();
-                while (c->allocs.size() > kept) {
-                    cudaFreeAsync(c->allocs.back(), s);
-                    c->allocs.pop_back();
-                }
+                wf_cache_free_allocs(*c, s, kept);
                 std::memset(&c->alt, 0, sizeof(c->alt));
             }
         }
         c->pool = pool;
         c->cap_mis = cap_mis;
         c->cap_sh = cap_sh;
+        ++c->builds;
     }
     out = c;
     return FM_OK;
@@ -1866,26 +1916,8 @@ fm_status wavefront_adjoint(fm_ctx* ctx, const std::vector<WfView>& views, const
 
 void wf_cache_release(fm_ctx* ctx)
 {
-    for (WfCache*& c : ctx->wf_cache) {
-        if (!c) continue;
-        wf_cache_drop_graph(*c);
-        wf_cache_free_state(*c, ctx->stream);
-        if (c->partial) cudaFreeAsync(c->partial, ctx->stream);
-        if (c->d_views) cudaFreeAsync(c->d_views, ctx->stream);
-        if (c->cnt) cudaFreeAsync(c->cnt, ctx->stream);
-        cudaStreamSynchronize(ctx->stream);
-        if (c->h_views) cudaFreeHost(c->h_views);
-        if (c->h_block) cudaFreeHost(c->h_block);
-        for (cudaStream_t x : c->side)
-            if (x) cudaStreamDestroy(x);
-        for (cudaEvent_t ev : {c->fork, c->fork2, c->join[0], c->join[1]})
-            if (ev) cudaEventDestroy(ev);
-        if (c->e0) cudaEventDestroy(c->e0);
-        if (c->e1) cudaEventDestroy(c->e1);
-        for (cudaEvent_t ev : c->pev) cudaEventDestroy(ev);
-        delete c;
-        c = nullptr;
-    }
+    for (WfCache*& c : ctx->wf_cache)
+        if (c) wf_cache_destroy(c, ctx->stream);
 }
 
 fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& cam, const RenderCfg& cfg, float* rgb,
@@ -1918,3 +1950,18 @@ fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& 
 }
 
 }  // namespace fm
+
+// Used by tests: bounds the device memory of each of the context's workspaces (0: by the
+// device only), and reports the forward one's device bytes, how often its state was
+// allocated and whether it has the second set of ray records.
+extern "C" void fm_internal_limit_workspace(fm_ctx* ctx, int64_t bytes)
+{
+    if (ctx) ctx->wf_limit = bytes > 0 ? (size_t)bytes : 0;
+}
+extern "C" void fm_internal_workspace(const fm_ctx* ctx, int64_t* out)
+{
+    const fm::WfCache* c = ctx ? ctx->wf_cache[0] : nullptr;
+    out[0] = c ? (int64_t)c->held : 0;
+    out[1] = c ? c->builds : 0;
+    out[2] = c && c->alt.mis_o ? 1 : 0;
+}

@@ -1,0 +1,108 @@
+"""Renders on a device that is short of memory: an allocation refused at each place where the
+wavefront workspace grows is an error or a smaller workspace, never a broken context.  The
+refusals come from a bound on what a context's workspace may hold, not from a full device."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import fumeng_b200 as fb
+from fumeng_b200 import synth
+
+SPECS = [synth.material_scene(3, res=96), synth.cornell(res=100, spp=9)]
+
+
+class _Ctx:
+    """A context of its own, with the bound and what the workspace holds."""
+
+    def __enter__(self):
+        self.ctx = fb.Context(0)
+        self.scenes = []
+        return self
+
+    def __exit__(self, *a):
+        for s in self.scenes:
+            s.destroy()
+        self.ctx.close()
+
+    def scene(self, spec):
+        self.scenes.append(self.ctx.create_scene(spec.to_desc()))
+        return self.scenes[-1]
+
+    def limit(self, nbytes):
+        self.ctx.lib.fm_internal_limit_workspace(self.ctx.h, C.c_int64(nbytes))
+
+    def workspace(self):
+        """(device bytes, times the state was allocated, second set of ray records)."""
+        out = (C.c_int64 * 3)()
+        self.ctx.lib.fm_internal_workspace(self.ctx.h, out)
+        return tuple(out)
+
+    def batch(self, pool=1 << 16, spp=20):
+        if not self.scenes:
+            for s in SPECS:
+                self.scene(s)
+        return self.ctx.render_batch(self.scenes, [s.camera_struct() for s in SPECS],
+                                     [s.render_params(spp=spp, seed=5) for s in SPECS], want_aov=True,
+                                     tuning=fb.Tuning(pool, 128, 128, 4, 0, 0))
+
+
+def _counts(stats):
+    return stats.paths, stats.closest_rays, stats.shadow_rays, stats.bounces
+
+
+def _same(a, b):
+    """Images that differ only in the order of float additions, and equal ray counts."""
+    assert _counts(a[3]) == _counts(b[3])
+    for x, y in zip(a[:3], b[:3]):
+        for p, q in zip(x, y):
+            np.testing.assert_allclose(p, q, rtol=1e-5, atol=1e-6)
+
+
+@pytest.fixture(scope="module")
+def unlimited(fm_lib):
+    with _Ctx() as c:
+        images = c.batch()
+        return images, c.workspace()
+
+
+@pytest.mark.gpu
+def test_a_workspace_that_could_not_be_made_is_made_later(unlimited):
+    with _Ctx() as c:
+        c.limit(1)
+        for _ in range(2):
+            with pytest.raises(fb.FumengError) as e:
+                c.batch()
+            assert e.value.status == fb.FM_ERR_OOM
+            assert c.workspace() == (0, 0, 0)
+        c.limit(0)
+        _same(c.batch(), unlimited[0])
+
+
+@pytest.mark.gpu
+def test_a_refused_larger_pool_leaves_the_context_usable(unlimited):
+    with _Ctx() as c:
+        c.batch(pool=1 << 15)
+        c.limit(2 * c.workspace()[0])
+        for _ in range(2):
+            with pytest.raises(fb.FumengError) as e:
+                c.batch(pool=1 << 18, spp=80)
+            assert e.value.status == fb.FM_ERR_OOM
+        _same(c.batch(pool=1 << 15), unlimited[0])
+        c.limit(0)
+        _same(c.batch(), unlimited[0])
+
+
+@pytest.mark.gpu
+def test_renders_with_one_set_of_ray_records(unlimited):
+    """Without room for the second set, the MIS and shadow rays of an iteration are resolved
+    before shading queues the next ones into the same records."""
+    images, (held, builds, second) = unlimited
+    assert (builds, second) == (1, 1)
+    with _Ctx() as c:
+        c.limit(held - 1)
+        got = c.batch()
+        assert c.workspace()[1:] == (1, 0) and c.workspace()[0] < held
+        _same(got, images)
+        _same(c.batch(), images)
+        assert c.workspace()[1:] == (1, 0)
