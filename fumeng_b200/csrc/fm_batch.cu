@@ -127,17 +127,12 @@ fm_status autotune(fm_ctx* ctx, int32_t n, const fm_scene* const* scenes, const 
     // Pools up to 2^25 slots: on the 64-scene batch (250 M paths) a render ran 368 /
     // 333 / 302 / 307 ms at 2^22 / 2^24 / 2^25 / 2^26 slots -- a larger pool means fewer
     // wavefront iterations, so fewer launches and fewer kernel tails.  A candidate's
-    // workspace (about 332 B plus 100 B per light and direct-lighting round per slot) must
-    // fit in half of the device memory free now.
-    int max_rays = 1;
-    for (const auto& v : views) max_rays = std::max(max_rays, v.num_lights * v.cfg.direct_loop);
+    // workspace must fit in half of the device memory free now.
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         free_b = 0;
     }
-    const double slot_bytes = 332.0 + 100.0 * max_rays + 64.0;
-    const double pool_cap = 0.5 * (double)free_b / slot_bytes;
     // warm-up, then coordinate descent over pool size, trace block, shade block, graph depth
     st = trial(best);
     best_rate = -1.0;
@@ -145,7 +140,7 @@ fm_status autotune(fm_ctx* ctx, int32_t n, const fm_scene* const* scenes, const 
                              (int64_t)1 << 23, (int64_t)1 << 24, (int64_t)1 << 25};
     for (int64_t p : pools) {
         if (st != FM_OK) break;
-        if (((double)p > samples * 2.0 || (double)p > pool_cap) && p != pools[0]) continue;
+        if (((double)p > samples * 2.0 || wavefront_bytes(views, p) > free_b / 2) && p != pools[0]) continue;
         fm_tuning t = best;
         t.pool = p;
         st = trial(t);

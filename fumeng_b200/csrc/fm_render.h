@@ -71,6 +71,8 @@ fm_status reduce_views(fm_ctx* ctx, const std::vector<WfView>& views);
 // Renders several views (possibly of different scenes) in one wavefront.
 fm_status wavefront_views(fm_ctx* ctx, const std::vector<WfView>& views, const WfTuning& tune, Counters* cnt,
                           WfTimes* times);
+// Device bytes of the workspace of such a render with `pool` path slots.
+size_t wavefront_bytes(std::vector<WfView> views, int64_t pool);
 // Path-replay adjoint over views of one scene: gradients of sum(drgb * image) with
 // respect to texture texels and material constants.  rgb (if set) receives the primal
 // image of the same samples.

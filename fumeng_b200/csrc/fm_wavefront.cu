@@ -1438,6 +1438,108 @@ void wf_cache_free_state(WfCache& c, cudaStream_t s)
     c.pool = c.cap_mis = c.cap_sh = 0;
 }
 
+// Calls f(pointer, count) for every buffer of a set of ray records ...
+template <class F>
+void each_ray_buffer(RayQueue& r, int64_t cap_mis, int64_t cap_sh, F&& f)
+{
+    f(r.mis_o, cap_mis);
+    f(r.mis_d, cap_mis);
+    f(r.mis_a, cap_mis);
+    f(r.sh_o, cap_sh);
+    f(r.sh_d, cap_sh);
+    f(r.sh_c, cap_sh);
+}
+// ... and of the state of `pool` path slots (one set of ray records included).
+template <class F>
+void each_state_buffer(WfState& b, bool adj, int64_t pool, int64_t cap_mis, int64_t cap_sh, F&& f)
+{
+    f(b.next_item, 1);
+    f(b.item, pool);
+    f(b.k, pool);
+    f(b.view, pool);
+    f(b.flags, pool);
+    f(b.rng, pool);
+    f(b.beta, pool);
+    f(b.col, pool);
+    f(b.ro, pool);
+    f(b.rd, pool);
+    f(b.hit, pool);
+    f(b.acc, pool);
+    f(b.isum, pool);
+    f(b.icomp, pool);
+    f(b.asum, pool);
+    f(b.nsum, pool);
+    f(b.cont_q, pool);
+    f(b.cont_h, pool);
+    f(b.cont_v, pool);
+    f(b.disney_q, pool);
+    f(b.simple_q, pool);
+    each_ray_buffer(b.rq, cap_mis, cap_sh, f);
+    f(b.mis_h, cap_mis);
+    f(b.sh_h, cap_sh);
+    f(b.qc, kQcCount);
+    f(b.tspan, 4);
+    if (adj) {
+        f(b.disney_r, pool);
+        f(b.simple_r, pool);
+        f(b.lp, pool);
+        f(b.dfr, 5 * pool);
+        f(b.vg, 2 * pool);
+        f(b.gq, 6 * pool);
+        f(b.sh_g, 3 * cap_sh);
+        f(b.mis_g, 8 * cap_mis);
+    }
+}
+
+// What a render of some views needs of the workspace at a tuning's pool.
+struct WfSizes {
+    int64_t pool = 0, cap_mis = 0, cap_sh = 0;
+    int64_t items = 0, partial_f4 = 0;
+    double samples = 0.0;
+    bool aov = false;   // some view wants albedo or normal images
+};
+
+// Sizes a render and splits the views' samples into work items: about four per path slot
+// over the whole job.  Albedo and normal sums are kept, and their partial sums written, only
+// when asked for (they are a third of a path's state traffic).
+WfSizes size_views(std::vector<WfView>& views, int64_t tune_pool)
+{
+    WfSizes z;
+    int64_t max_lights = 1, max_dl = 1;
+    for (const auto& v : views) {
+        z.aov = z.aov || v.alb || v.nrm;
+        z.samples += (double)v.cfg.width * v.cfg.height * v.cfg.spp;
+        max_dl = std::max<int64_t>(max_dl, v.cfg.direct_loop);
+        max_lights = std::max<int64_t>(max_lights, v.num_lights);
+    }
+    z.pool = std::max<int64_t>(1024, std::min<int64_t>(tune_pool, (int64_t)z.samples));
+    z.cap_mis = z.pool * max_dl;
+    z.cap_sh = z.pool * max_dl * max_lights;
+    const double per_item = z.samples / (4.0 * (double)z.pool);
+    for (auto& v : views) {
+        const int chunk = (int)std::floor(per_item);
+        v.chunk = std::max(1, std::min(chunk, v.cfg.spp));
+        v.nchunks = (v.cfg.spp + v.chunk - 1) / v.chunk;
+        v.item_base = z.items;
+        const int64_t items = (int64_t)v.cfg.width * v.cfg.height * v.nchunks;
+        z.items += items;
+        v.partial_f4 = z.aov ? 3 : 1;
+        z.partial_f4 += v.partial_f4 * items;
+    }
+    return z;
+}
+
+// Device bytes of the forward workspace for such a render, both sets of ray records included.
+size_t forward_bytes(const WfSizes& z)
+{
+    size_t total = sizeof(float4) * (size_t)z.partial_f4;
+    auto add = [&](auto*& p, size_t count) { total += sizeof(*p) * count; };
+    WfState b;
+    each_state_buffer(b, false, z.pool, z.cap_mis, z.cap_sh, add);
+    each_ray_buffer(b.rq, z.cap_mis, z.cap_sh, add);
+    return total;
+}
+
 // Releases a workspace, complete or not.
 void wf_cache_destroy(WfCache*& c, cudaStream_t s)
 {
@@ -1520,7 +1622,6 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
         cap_mis = std::max(cap_mis, c->cap_mis);
         cap_sh = std::max(cap_sh, c->cap_sh);
         wf_cache_free_state(*c, s);
-        WfState& b = c->bufs;
         bool ok = true;
         auto A = [&](auto*& p, size_t count) {
             void* q = nullptr;
@@ -1532,50 +1633,7 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
                 ok = false;
             }
         };
-        A(b.next_item, 1);
-        A(b.item, pool);
-        A(b.k, pool);
-        A(b.view, pool);
-        A(b.flags, pool);
-        A(b.rng, pool);
-        A(b.beta, pool);
-        A(b.col, pool);
-        A(b.ro, pool);
-        A(b.rd, pool);
-        A(b.hit, pool);
-        A(b.acc, pool);
-        A(b.isum, pool);
-        A(b.icomp, pool);
-        A(b.asum, pool);
-        A(b.nsum, pool);
-        A(b.cont_q, pool);
-        A(b.cont_h, pool);
-        A(b.cont_v, pool);
-        A(b.disney_q, pool);
-        A(b.simple_q, pool);
-        auto queue = [&](RayQueue& r) {
-            A(r.mis_o, cap_mis);
-            A(r.mis_d, cap_mis);
-            A(r.mis_a, cap_mis);
-            A(r.sh_o, cap_sh);
-            A(r.sh_d, cap_sh);
-            A(r.sh_c, cap_sh);
-        };
-        queue(b.rq);
-        A(b.mis_h, cap_mis);
-        A(b.sh_h, cap_sh);
-        A(b.qc, kQcCount);
-        A(b.tspan, 4);
-        if (adj) {
-            A(b.disney_r, pool);
-            A(b.simple_r, pool);
-            A(b.lp, pool);
-            A(b.dfr, 5 * (size_t)pool);
-            A(b.vg, 2 * (size_t)pool);
-            A(b.gq, 3 * 2 * (size_t)pool);
-            A(b.sh_g, 3 * (size_t)cap_sh);
-            A(b.mis_g, 8 * (size_t)cap_mis);
-        }
+        each_state_buffer(c->bufs, adj, pool, cap_mis, cap_sh, A);
         if (!ok) {
             cudaGetLastError();
             wf_cache_free_state(*c, s);
@@ -1584,7 +1642,7 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
         if (!adj) {
             // the second set of ray records; without room for it renders run with one
             const size_t kept = c->allocs.size();
-            queue(c->alt);
+            each_ray_buffer(c->alt, cap_mis, cap_sh, A);
             if (!ok) {
                 cudaGetLastError();
                 wf_cache_free_allocs(*c, s, kept);
@@ -1606,35 +1664,10 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
 {
     cudaStream_t s = ctx->stream;
     std::vector<WfView> views = views_in;
-    // samples per work item: aim for ~4 items per path slot over the whole job
-    double total_samples = 0.0;
-    int max_lights = 1, max_dl = 1;
-    // albedo and normal sums are kept, and their partial sums written, only when asked for
-    // (they are a third of a path's state traffic)
-    bool aov = false;
-    for (const auto& v : views) aov = aov || v.alb || v.nrm;
-    for (const auto& v : views) {
-        total_samples += (double)v.cfg.width * v.cfg.height * v.cfg.spp;
-        max_dl = std::max(max_dl, v.cfg.direct_loop);
-        max_lights = std::max(max_lights, v.num_lights);
-    }
-    const int64_t pool = std::max<int64_t>(1024, std::min<int64_t>(tune.pool, (int64_t)total_samples));
-    const double per_item = total_samples / (4.0 * (double)pool);
-    int64_t item_base = 0, partial_f4 = 0;
-    for (auto& v : views) {
-        int chunk = (int)std::floor(per_item);
-        chunk = std::max(1, std::min(chunk, v.cfg.spp));
-        v.chunk = chunk;
-        v.nchunks = (v.cfg.spp + chunk - 1) / chunk;
-        v.item_base = item_base;
-        const int64_t npix = (int64_t)v.cfg.width * v.cfg.height;
-        item_base += npix * v.nchunks;
-        v.partial_f4 = aov ? 3 : 1;
-        partial_f4 += v.partial_f4 * npix * v.nchunks;
-    }
+    const WfSizes z = size_views(views, tune.pool);
+    const int64_t pool = z.pool;
     WfCache* c = nullptr;
-    fm_status result = wf_cache_reserve(ctx, ADJ, pool, pool * max_dl, pool * max_dl * (int64_t)max_lights, partial_f4,
-                                        (int32_t)views.size(), c);
+    fm_status result = wf_cache_reserve(ctx, ADJ, pool, z.cap_mis, z.cap_sh, z.partial_f4, (int32_t)views.size(), c);
     if (result != FM_OK) return result;
     {
         float4* p = c->partial;
@@ -1648,11 +1681,11 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     std::memcpy(&st, &c->bufs, sizeof(st));
     st.pool = pool;
     st.nviews = (int32_t)views.size();
-    st.aov = aov ? 1 : 0;
-    st.total_items = item_base;
+    st.aov = z.aov ? 1 : 0;
+    st.total_items = z.items;
     st.cap_cont = pool;
-    st.cap_mis = pool * max_dl;
-    st.cap_sh = pool * max_dl * (int64_t)max_lights;
+    st.cap_mis = z.cap_mis;
+    st.cap_sh = z.cap_sh;
     if (tune.queue_limit > 0) {
         // below the allocated capacities: appends beyond them are counted and dropped
         st.cap_cont = std::min<int64_t>(st.cap_cont, tune.queue_limit);
@@ -1715,7 +1748,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
         max_chunk = std::max(max_chunk, v.chunk);
     }
     const double iter_bound =
-        (total_samples / (double)pool + 4.0 * max_chunk + 8.0) * (max_depth + 2) * 4.0 * (ADJ ? 2.0 : 1.0) + 1000.0;
+        (z.samples / (double)pool + 4.0 * max_chunk + 8.0) * (max_depth + 2) * 4.0 * (ADJ ? 2.0 : 1.0) + 1000.0;
     int64_t max_launches = (int64_t)(iter_bound / body_iters) + 16;
     if (tune.max_iterations > 0)
         max_launches = std::min<int64_t>(max_launches, (tune.max_iterations + body_iters - 1) / body_iters);
@@ -1920,6 +1953,11 @@ void wf_cache_release(fm_ctx* ctx)
         if (c) wf_cache_destroy(c, ctx->stream);
 }
 
+size_t wavefront_bytes(std::vector<WfView> views, int64_t pool) { return forward_bytes(size_views(views, pool)); }
+
+// The most device memory that fm_render's workspace takes for more than the default slots.
+constexpr size_t kWideBytes = size_t(8000) * 1000 * 1000;
+
 fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& cam, const RenderCfg& cfg, float* rgb,
                            float* alb, float* nrm, Counters* cnt)
 {
@@ -1938,9 +1976,8 @@ fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& 
     // the workspace stays below 8 GB and fits.
     WfTuning t;
     const double samples = (double)cfg.width * cfg.height * cfg.spp;
-    const double slot_bytes = 332.0 + 100.0 * std::max(1, v.num_lights) * cfg.direct_loop;
     for (int64_t pool = (int64_t)1 << 23; pool > t.pool; pool /= 2) {
-        if (samples < 1.5 * (double)pool || slot_bytes * (double)pool > 8e9) continue;
+        if (samples < 1.5 * (double)pool || wavefront_bytes({v}, pool) > kWideBytes) continue;
         WfTuning wide;
         wide.pool = pool;
         const fm_status st = wavefront_views(ctx, {v}, wide, cnt, nullptr);

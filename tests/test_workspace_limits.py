@@ -106,3 +106,17 @@ def test_renders_with_one_set_of_ray_records(unlimited):
         _same(got, images)
         _same(c.batch(), images)
         assert c.workspace()[1:] == (1, 0)
+
+
+@pytest.mark.gpu
+def test_direct_lighting_rounds_count_towards_the_bound_of_a_wide_pool(fm_lib):
+    """13.6 M samples would have 2^23 slots, whose ray records for six rounds take 12.5 GB."""
+    with _Ctx() as c:
+        spec = synth.cornell(res=1024)
+        sc = c.scene(spec)
+        p = spec.render_params(spp=13, seed=1)
+        p.depth, p.direct_loop = 1, 6
+        st = sc.render(spec.camera_struct(), p, want_aov=False)[3]
+        assert st.paths == 1024 * 1024 * 13
+        held = c.workspace()[0]
+        assert 6e9 < held <= 8e9   # 2^22 slots
