@@ -1955,8 +1955,46 @@ void wf_cache_release(fm_ctx* ctx)
 
 size_t wavefront_bytes(std::vector<WfView> views, int64_t pool) { return forward_bytes(size_views(views, pool)); }
 
+namespace {
+
 // The most device memory that fm_render's workspace takes for more than the default slots.
 constexpr size_t kWideBytes = size_t(8000) * 1000 * 1000;
+
+// Whether a render of more than the default slots has its workspace already or may let it
+// grow: within kWideBytes, and within half of the memory that is free or that the workspace
+// and the device's memory pool hold and would use again.  Asked before the present workspace
+// is given up, so a pool that does not fit costs nothing, not even the kept graph.  A size
+// that was refused all the same (another process took the memory) is not tried again.
+bool wide_pool_fits(fm_ctx* ctx, const WfSizes& z)
+{
+    if (ctx->wf_refused > 0 && z.pool >= ctx->wf_refused) return false;
+    const WfCache* c = ctx->wf_cache[0];
+    WfSizes need = z;
+    size_t held = 0;
+    if (c) {
+        if (z.pool <= c->pool && z.cap_mis <= c->cap_mis && z.cap_sh <= c->cap_sh && z.partial_f4 <= c->partial_f4)
+            return true;
+        need.pool = std::max(z.pool, c->pool);
+        need.cap_mis = std::max(z.cap_mis, c->cap_mis);
+        need.cap_sh = std::max(z.cap_sh, c->cap_sh);
+        need.partial_f4 = std::max(z.partial_f4, c->partial_f4);
+        held = c->held;
+    }
+    const size_t bytes = forward_bytes(need);
+    if (bytes > kWideBytes) return false;
+    size_t free_b = 0, total_b = 0;
+    uint64_t reserved = 0, used = 0;
+    cudaMemPool_t mem;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || cudaDeviceGetDefaultMemPool(&mem, ctx->device) != cudaSuccess ||
+        cudaMemPoolGetAttribute(mem, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(mem, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes <= (free_b + (size_t)(reserved - std::min(reserved, used)) + held) / 2;
+}
+
+}  // namespace
 
 fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& cam, const RenderCfg& cfg, float* rgb,
                            float* alb, float* nrm, Counters* cnt)
@@ -1973,15 +2011,20 @@ fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& 
     // slot -- more slots mean fewer iterations, so fewer launches and kernel tails
     // (1920x1080 through 1.3 M triangles with 2^21 / 2^22 / 2^23 / 2^24 slots: 5.76 / 5.49 /
     // 5.49 / 5.51 ms at 4 samples per pixel, 18.8 / 17.3 / 16.8 / 17.3 ms at 16) -- as long as
-    // the workspace stays below 8 GB and fits.
+    // the device has room for their workspace.
     WfTuning t;
     const double samples = (double)cfg.width * cfg.height * cfg.spp;
     for (int64_t pool = (int64_t)1 << 23; pool > t.pool; pool /= 2) {
-        if (samples < 1.5 * (double)pool || wavefront_bytes({v}, pool) > kWideBytes) continue;
+        if (samples < 1.5 * (double)pool) continue;
+        std::vector<WfView> views{v};
+        if (!wide_pool_fits(ctx, size_views(views, pool))) continue;
         WfTuning wide;
         wide.pool = pool;
+        const std::string before = ctx->error;
         const fm_status st = wavefront_views(ctx, {v}, wide, cnt, nullptr);
         if (st != FM_ERR_OOM) return st;
+        ctx->error = before;
+        ctx->wf_refused = pool;
     }
     return wavefront_views(ctx, {v}, t, cnt, nullptr);
 }
@@ -1993,7 +2036,9 @@ fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& 
 // allocated and whether it has the second set of ray records.
 extern "C" void fm_internal_limit_workspace(fm_ctx* ctx, int64_t bytes)
 {
-    if (ctx) ctx->wf_limit = bytes > 0 ? (size_t)bytes : 0;
+    if (!ctx) return;
+    ctx->wf_limit = bytes > 0 ? (size_t)bytes : 0;
+    ctx->wf_refused = 0;
 }
 extern "C" void fm_internal_workspace(const fm_ctx* ctx, int64_t* out)
 {

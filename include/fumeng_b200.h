@@ -222,7 +222,7 @@ typedef struct {
  * of which there are about four to eight per slot; more for adjoint renders; pinned staging;
  * the instantiated render graph) and releases it in fm_ctx_destroy.  fm_render uses 2^21
  * slots, or up to 2^23 where a render has 1.5 samples or more per slot and the workspace
- * stays below 8 GB. */
+ * stays below 8 GB and half of the device memory it finds free. */
 fm_status fm_ctx_create(int device, fm_ctx** out);
 void fm_ctx_destroy(fm_ctx* ctx);
 const char* fm_last_error(const fm_ctx* ctx);

@@ -120,3 +120,39 @@ def test_direct_lighting_rounds_count_towards_the_bound_of_a_wide_pool(fm_lib):
         assert st.paths == 1024 * 1024 * 13
         held = c.workspace()[0]
         assert 6e9 < held <= 8e9   # 2^22 slots
+
+
+@pytest.mark.gpu
+def test_a_wide_pool_that_does_not_fit_is_tried_once(fm_lib):
+    """7.3 M samples have 2^22 slots.  Where those are refused, the render runs with the default
+    ones, reports no error, and later renders keep the workspace (and its graph)."""
+    spec = synth.cornell(res=1024)
+    cam = spec.camera_struct()
+    few, many = spec.render_params(spp=3, seed=1), spec.render_params(spp=7, seed=2)
+    with _Ctx() as c:
+        sc = c.scene(spec)
+        want = sc.render(cam, many, want_aov=False)
+        wide = c.workspace()
+        for _ in range(2):
+            sc.render(cam, many, want_aov=False)
+            sc.render(cam, few, want_aov=False)
+        assert c.workspace() == wide and wide[1] == 1
+    with _Ctx() as c:
+        sc = c.scene(spec)
+        sc.render(cam, few, want_aov=False)
+        narrow = c.workspace()
+        assert narrow[0] < 0.6 * wide[0]
+        c.limit(int(1.3 * narrow[0]))
+        got = sc.render(cam, many, want_aov=False)
+        assert c.ctx.lib.fm_last_error(c.ctx.h) == b""
+        assert _counts(got[3]) == _counts(want[3])
+        np.testing.assert_allclose(got[0], want[0], rtol=1e-5, atol=1e-6)
+        after = c.workspace()
+        assert after[1:] == (2, 1)
+        for _ in range(2):
+            sc.render(cam, many, want_aov=False)
+            sc.render(cam, few, want_aov=False)
+        assert c.workspace() == after
+        c.limit(0)
+        sc.render(cam, many, want_aov=False)
+        assert c.workspace()[0] > 0.9 * wide[0]
