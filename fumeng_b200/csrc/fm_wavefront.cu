@@ -90,10 +90,11 @@ struct WfState {
     float4* rd;
     float4* hit;
     float4* acc;          // adjoint renders: the iteration's MIS, shadow and emission contributions
-                          // (atomic adds from the resolve kernels; forward renders add them to col)
+                          // (atomic adds from the resolve kernels; forward renders add them to col
+                          // and have none)
     float4* isum;
     float4* icomp;
-    float4* asum;
+    float4* asum;         // where aov is set (null otherwise)
     float4* nsum;
     // queues
     int32_t* cont_q;
@@ -1313,7 +1314,7 @@ __global__ void k_wf_init(WfState st)
     if (blockIdx.x == 0 && threadIdx.x == 0) st.tspan[0] = ~0ull;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < st.pool; s += (int64_t)gridDim.x * blockDim.x) {
         st.flags[s] = kNeedItem;
-        st.acc[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (st.acc) st.acc[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         st.col[s] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
@@ -1363,6 +1364,8 @@ __global__ void k_counters_add(Counters* dst, const Counters* src)
 struct WfCache {
     bool adj = false;
     int64_t pool = 0, cap_mis = 0, cap_sh = 0, partial_f4 = 0;
+    int64_t aov_pool = 0;        // capacity of asum and nsum, which only some renders need
+    float4 *asum = nullptr, *nsum = nullptr;
     int32_t nviews = 0;
     size_t held = 0;             // device bytes of everything below
     int64_t builds = 0;          // times the state buffers were allocated
@@ -1438,6 +1441,14 @@ void wf_cache_free_state(WfCache& c, cudaStream_t s)
     c.pool = c.cap_mis = c.cap_sh = 0;
 }
 
+void wf_cache_free_aov(WfCache& c, cudaStream_t s)
+{
+    wf_free(c, s, c.asum, sizeof(float4) * (size_t)c.aov_pool);
+    wf_free(c, s, c.nsum, sizeof(float4) * (size_t)c.aov_pool);
+    c.asum = c.nsum = nullptr;
+    c.aov_pool = 0;
+}
+
 // Calls f(pointer, count) for every buffer of a set of ray records ...
 template <class F>
 void each_ray_buffer(RayQueue& r, int64_t cap_mis, int64_t cap_sh, F&& f)
@@ -1464,11 +1475,8 @@ void each_state_buffer(WfState& b, bool adj, int64_t pool, int64_t cap_mis, int6
     f(b.ro, pool);
     f(b.rd, pool);
     f(b.hit, pool);
-    f(b.acc, pool);
     f(b.isum, pool);
     f(b.icomp, pool);
-    f(b.asum, pool);
-    f(b.nsum, pool);
     f(b.cont_q, pool);
     f(b.cont_h, pool);
     f(b.cont_v, pool);
@@ -1480,6 +1488,7 @@ void each_state_buffer(WfState& b, bool adj, int64_t pool, int64_t cap_mis, int6
     f(b.qc, kQcCount);
     f(b.tspan, 4);
     if (adj) {
+        f(b.acc, pool);
         f(b.disney_r, pool);
         f(b.simple_r, pool);
         f(b.lp, pool);
@@ -1496,7 +1505,7 @@ struct WfSizes {
     int64_t pool = 0, cap_mis = 0, cap_sh = 0;
     int64_t items = 0, partial_f4 = 0;
     double samples = 0.0;
-    bool aov = false;   // some view wants albedo or normal images
+    int64_t aov_pool = 0;   // slots with albedo and normal sums: `pool`, or 0 when no view wants those images
 };
 
 // Sizes a render and splits the views' samples into work items: about four per path slot
@@ -1506,13 +1515,15 @@ WfSizes size_views(std::vector<WfView>& views, int64_t tune_pool)
 {
     WfSizes z;
     int64_t max_lights = 1, max_dl = 1;
+    bool aov = false;
     for (const auto& v : views) {
-        z.aov = z.aov || v.alb || v.nrm;
+        aov = aov || v.alb || v.nrm;
         z.samples += (double)v.cfg.width * v.cfg.height * v.cfg.spp;
         max_dl = std::max<int64_t>(max_dl, v.cfg.direct_loop);
         max_lights = std::max<int64_t>(max_lights, v.num_lights);
     }
     z.pool = std::max<int64_t>(1024, std::min<int64_t>(tune_pool, (int64_t)z.samples));
+    z.aov_pool = aov ? z.pool : 0;
     z.cap_mis = z.pool * max_dl;
     z.cap_sh = z.pool * max_dl * max_lights;
     const double per_item = z.samples / (4.0 * (double)z.pool);
@@ -1523,7 +1534,7 @@ WfSizes size_views(std::vector<WfView>& views, int64_t tune_pool)
         v.item_base = z.items;
         const int64_t items = (int64_t)v.cfg.width * v.cfg.height * v.nchunks;
         z.items += items;
-        v.partial_f4 = z.aov ? 3 : 1;
+        v.partial_f4 = aov ? 3 : 1;
         z.partial_f4 += v.partial_f4 * items;
     }
     return z;
@@ -1537,7 +1548,12 @@ size_t forward_bytes(const WfSizes& z)
     WfState b;
     each_state_buffer(b, false, z.pool, z.cap_mis, z.cap_sh, add);
     each_ray_buffer(b.rq, z.cap_mis, z.cap_sh, add);
-    return total;
+    return total + 2 * sizeof(float4) * (size_t)z.aov_pool;
+}
+
+bool wf_state_holds(const WfCache& c, const WfSizes& z)
+{
+    return z.pool <= c.pool && z.cap_mis <= c.cap_mis && z.cap_sh <= c.cap_sh;
 }
 
 // Releases a workspace, complete or not.
@@ -1545,6 +1561,7 @@ void wf_cache_destroy(WfCache*& c, cudaStream_t s)
 {
     wf_cache_drop_graph(*c);
     wf_cache_free_state(*c, s);
+    wf_cache_free_aov(*c, s);
     wf_free(*c, s, c->partial, sizeof(float4) * (size_t)c->partial_f4);
     wf_free(*c, s, c->d_views, sizeof(WfView) * (size_t)c->nviews);
     wf_free(*c, s, c->cnt, sizeof(Counters));
@@ -1560,9 +1577,8 @@ void wf_cache_destroy(WfCache*& c, cudaStream_t s)
     c = nullptr;
 }
 
-// Makes the workspace of `ctx` (forward or adjoint) hold at least the given capacities.
-fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis, int64_t cap_sh, int64_t partial_f4,
-                           int32_t nviews, WfCache*& out)
+// Makes the workspace of `ctx` (forward or adjoint) hold at least what a render needs.
+fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, const WfSizes& need, int32_t nviews, WfCache*& out)
 {
     cudaStream_t s = ctx->stream;
     WfCache*& c = ctx->wf_cache[adj ? 1 : 0];
@@ -1606,21 +1622,34 @@ fm_status wf_cache_reserve(fm_ctx* ctx, bool adj, int64_t pool, int64_t cap_mis,
         c->d_views = d;
         c->nviews = nviews;
     }
-    if (partial_f4 > c->partial_f4) {
+    if (need.partial_f4 > c->partial_f4) {
         wf_free(*c, s, c->partial, sizeof(float4) * (size_t)c->partial_f4);
         c->partial = nullptr;
         c->partial_f4 = 0;
-        if (wf_malloc(ctx, *c, (void**)&c->partial, sizeof(float4) * (size_t)partial_f4) != cudaSuccess) {
+        if (wf_malloc(ctx, *c, (void**)&c->partial, sizeof(float4) * (size_t)need.partial_f4) != cudaSuccess) {
             cudaGetLastError();
             return set_error(ctx, FM_ERR_OOM, "wavefront: partial buffer allocation failed");
         }
-        c->partial_f4 = partial_f4;
+        c->partial_f4 = need.partial_f4;
     }
-    if (pool > c->pool || cap_mis > c->cap_mis || cap_sh > c->cap_sh) {
+    if (need.aov_pool > c->aov_pool) {
         wf_cache_drop_graph(*c);
-        pool = std::max(pool, c->pool);
-        cap_mis = std::max(cap_mis, c->cap_mis);
-        cap_sh = std::max(cap_sh, c->cap_sh);
+        wf_cache_free_aov(*c, s);
+        const size_t bytes = sizeof(float4) * (size_t)need.aov_pool;
+        float4 *as = nullptr, *ns = nullptr;
+        if (wf_malloc(ctx, *c, (void**)&as, bytes) != cudaSuccess || wf_malloc(ctx, *c, (void**)&ns, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            wf_free(*c, s, as, bytes);
+            return set_error(ctx, FM_ERR_OOM, "wavefront: albedo and normal sums' allocation failed");
+        }
+        c->asum = as;
+        c->nsum = ns;
+        c->aov_pool = need.aov_pool;
+    }
+    if (!wf_state_holds(*c, need)) {
+        wf_cache_drop_graph(*c);
+        const int64_t pool = std::max(need.pool, c->pool), cap_mis = std::max(need.cap_mis, c->cap_mis);
+        const int64_t cap_sh = std::max(need.cap_sh, c->cap_sh);
         wf_cache_free_state(*c, s);
         bool ok = true;
         auto A = [&](auto*& p, size_t count) {
@@ -1667,7 +1696,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     const WfSizes z = size_views(views, tune.pool);
     const int64_t pool = z.pool;
     WfCache* c = nullptr;
-    fm_status result = wf_cache_reserve(ctx, ADJ, pool, z.cap_mis, z.cap_sh, z.partial_f4, (int32_t)views.size(), c);
+    fm_status result = wf_cache_reserve(ctx, ADJ, z, (int32_t)views.size(), c);
     if (result != FM_OK) return result;
     {
         float4* p = c->partial;
@@ -1681,7 +1710,9 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     std::memcpy(&st, &c->bufs, sizeof(st));
     st.pool = pool;
     st.nviews = (int32_t)views.size();
-    st.aov = z.aov ? 1 : 0;
+    st.aov = z.aov_pool > 0 ? 1 : 0;
+    st.asum = st.aov ? c->asum : nullptr;
+    st.nsum = st.aov ? c->nsum : nullptr;
     st.total_items = z.items;
     st.cap_cont = pool;
     st.cap_mis = z.cap_mis;
@@ -1972,12 +2003,12 @@ bool wide_pool_fits(fm_ctx* ctx, const WfSizes& z)
     WfSizes need = z;
     size_t held = 0;
     if (c) {
-        if (z.pool <= c->pool && z.cap_mis <= c->cap_mis && z.cap_sh <= c->cap_sh && z.partial_f4 <= c->partial_f4)
-            return true;
+        if (wf_state_holds(*c, z) && z.partial_f4 <= c->partial_f4 && z.aov_pool <= c->aov_pool) return true;
         need.pool = std::max(z.pool, c->pool);
         need.cap_mis = std::max(z.cap_mis, c->cap_mis);
         need.cap_sh = std::max(z.cap_sh, c->cap_sh);
         need.partial_f4 = std::max(z.partial_f4, c->partial_f4);
+        need.aov_pool = std::max(z.aov_pool, c->aov_pool);
         held = c->held;
     }
     const size_t bytes = forward_bytes(need);

@@ -216,10 +216,11 @@ typedef struct {
 /* Replaces: nothing in the reference (it has no device); creates the CUDA context
  * holder used by every other call.  A context keeps its wavefront workspace between
  * renders (path-state and queue buffers sized to the largest pool and queues seen: for
- * forward renders 220 B per path slot plus, for each direct-lighting round, 112 B and 100 B
- * per light, 2.2 GB at 2^22 slots, one round and two lights, of which 48 B and 48 B per light
- * are left out when memory is short; 16 B, with albedo or normal images 48 B, per work item,
- * of which there are about four to eight per slot; more for adjoint renders; pinned staging;
+ * forward renders 172 B per path slot plus, for each direct-lighting round, 112 B and 100 B
+ * per light, 2.0 GB at 2^22 slots, one round and two lights, of which 48 B and 48 B per light
+ * are left out when memory is short; 32 B per slot of renders with albedo or normal images;
+ * 16 B, with such images 48 B, per work item, of which there are about four to eight per
+ * slot; more for adjoint renders; pinned staging;
  * the instantiated render graph) and releases it in fm_ctx_destroy.  fm_render uses 2^21
  * slots, or up to 2^23 where a render has 1.5 samples or more per slot and the workspace
  * stays below 8 GB and half of the device memory it finds free. */

@@ -156,3 +156,28 @@ def test_a_wide_pool_that_does_not_fit_is_tried_once(fm_lib):
         c.limit(0)
         sc.render(cam, many, want_aov=False)
         assert c.workspace()[0] > 0.9 * wide[0]
+
+
+@pytest.mark.gpu
+def test_albedo_and_normal_sums_are_held_once_they_are_asked_for(fm_lib):
+    spec = synth.material_scene(3, res=96)
+    cam, p = spec.camera_struct(), spec.render_params(spp=20, seed=3)
+    slots = 96 * 96 * 20
+    with _Ctx() as c, _Ctx() as fresh:
+        sc = c.scene(spec)
+        plain = sc.render(cam, p, want_aov=False)
+        lean, builds, _ = c.workspace()
+        got = sc.render(cam, p, want_aov=True)
+        full = c.workspace()
+        assert builds == full[1] == 1   # beside the state, which stays
+        # 32 B of sums per slot, and 32 B of partial sums per work item (four or more per slot,
+        # or one per sample)
+        assert full[0] - lean >= 64 * slots
+        again = sc.render(cam, p, want_aov=False)
+        assert c.workspace() == full
+        want = fresh.scene(spec).render(cam, p, want_aov=True)
+        for x in (plain, got, again):
+            assert _counts(x[3]) == _counts(want[3])
+            np.testing.assert_allclose(x[0], want[0], rtol=1e-5, atol=1e-6)
+        for k in (1, 2):
+            np.testing.assert_allclose(got[k], want[k], rtol=1e-5, atol=1e-6)
