@@ -246,36 +246,70 @@ void add_doubles(fm_ctx* ctx, double* dst, const double* src, size_t n)
 
 }  // namespace
 
-cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies)
+namespace {
+
+// Memory that only the host sees goes through the ring.  Page-locked memory the copy engine
+// reaches by itself, and memory of a device the host must not touch: both are left to
+// cudaMemcpyAsync.
+bool is_pageable(const void* p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
+// The copies that go through the ring: those that can, when they are kRingBytes in all.
+template <class Copy, class Can>
+void split_copies(const std::vector<Copy>& copies, std::vector<Copy>& ring, std::vector<Copy>& plain, Can&& can)
 {
     size_t total = 0;
-    for (const InCopy& c : copies) total += c.bytes;
-    if (total < kRingBytes) {
-        for (const InCopy& c : copies) {
-            const cudaError_t e = cudaMemcpyAsync(c.dst_dev, c.src_host, c.bytes, cudaMemcpyHostToDevice, s);
-            if (e != cudaSuccess) return e;
+    for (const Copy& c : copies) total += c.bytes;
+    if (total >= kRingBytes) {
+        total = 0;
+        for (const Copy& c : copies) {
+            const bool r = can(c);
+            (r ? ring : plain).push_back(c);
+            if (r) total += c.bytes;
         }
-        return cudaSuccess;
     }
-    const cudaError_t e = staging_ensure(ctx);
-    if (e != cudaSuccess) return e;
+    if (total >= kRingBytes) return;
+    ring.clear();
+    plain = copies;
+}
+
+}  // namespace
+
+cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies)
+{
+    std::vector<InCopy> ring, plain;
+    split_copies(copies, ring, plain, [](const InCopy& c) { return is_pageable(c.src_host); });
+    if (!ring.empty()) {
+        const cudaError_t e = staging_ensure(ctx);
+        if (e != cudaSuccess) return e;
+    }
+    for (const InCopy& c : plain) {
+        const cudaError_t e = cudaMemcpyAsync(c.dst_dev, c.src_host, c.bytes, cudaMemcpyHostToDevice, s);
+        if (e != cudaSuccess) return e;
+    }
+    if (ring.empty()) return cudaSuccess;
     Stager stager(ctx, s);
-    for (const InCopy& c : copies) stager.put(c.dst_dev, c.src_host, c.bytes);
+    for (const InCopy& c : ring) stager.put(c.dst_dev, c.src_host, c.bytes);
     stager.close();
     return stager.err;
 }
 
 cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies)
 {
-    size_t total = 0, added = 0;
-    for (const OutCopy& c : copies) {
-        total += c.bytes;
+    // sums are added by the host wherever they lie
+    std::vector<OutCopy> ring, plain;
+    split_copies(copies, ring, plain, [](const OutCopy& c) { return c.add || is_pageable(c.dst_host); });
+    size_t added = 0;
+    for (const OutCopy& c : plain)
         if (c.add) added += c.bytes / sizeof(double);
-    }
-    if (total >= kRingBytes) return copy_out(ctx, s, copies);
     std::vector<double> sums(added);
     size_t at = 0;
-    for (const OutCopy& c : copies) {
+    for (const OutCopy& c : plain) {
         void* dst = c.dst_host;
         if (c.add) {
             dst = sums.data() + at;
@@ -284,11 +318,12 @@ cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>
         const cudaError_t e = cudaMemcpyAsync(dst, c.src_dev, c.bytes, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return e;
     }
+    if (!ring.empty()) return copy_out(ctx, s, ring);
     if (added == 0) return cudaSuccess;
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
     at = 0;
-    for (const OutCopy& c : copies) {
+    for (const OutCopy& c : plain) {
         if (!c.add) continue;
         double* dst = static_cast<double*>(c.dst_host);
         for (size_t q = 0; q < c.bytes / sizeof(double); ++q) dst[q] += sums[at + q];

@@ -77,11 +77,13 @@ struct OutCopy {
 };
 cudaError_t copy_out(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies);
 
-// Host -> device copies of one call, stream-ordered on `s`; the host memory has been read
-// when it returns.  Below kRingBytes in all (a chunk) they are plain pageable copies: nothing
-// overlaps there, and waking the copy threads costs more than it saves (129,600 query
-// rays, 4.1 MB in and 1 MB out: 0.97 ms through the ring, 0.50 without).  Above it the ring
-// wins: a 1920x1080 post-process, 75 MB in and 43 MB out, 13.1 -> 8.2 ms.
+// Host -> device copies of one call, stream-ordered on `s`; the caller synchronises `s`
+// before it returns (a page-locked source is read until then).  Pageable memory goes through
+// the ring when it is kRingBytes in all (a chunk).  Below that nothing overlaps, and waking
+// the copy threads costs more than it saves (129,600 query rays, 4.1 MB in and 1 MB out: 0.97
+// ms through the ring, 0.50 without); above it the ring wins: a 1920x1080 post-process, 75 MB
+// in and 43 MB out, 13.1 -> 8.2 ms.  Memory that is page-locked already is copied from and to
+// directly.
 constexpr size_t kRingBytes = kStageChunk;
 struct InCopy {
     void* dst_dev;
@@ -90,8 +92,8 @@ struct InCopy {
 };
 cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies);
 
-// copy_out for a call's results: plain copies below kRingBytes in all, complete once the
-// caller has synchronised `s`.
+// copy_out for a call's results, by the same rule; complete once the caller has synchronised
+// `s`.
 cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies);
 
 }  // namespace fm
