@@ -259,9 +259,10 @@ bool is_pageable(const void* p)
     return false;
 }
 
-// The copies that go through the ring: those that can, when they are kRingBytes in all.
+// The copies that go through the ring: those that can, when they are kRingBytes in all and
+// there is page-locked memory for the ring (plain copies need none).
 template <class Copy, class Can>
-void split_copies(const std::vector<Copy>& copies, std::vector<Copy>& ring, std::vector<Copy>& plain, Can&& can)
+void split_copies(fm_ctx* ctx, const std::vector<Copy>& copies, std::vector<Copy>& ring, std::vector<Copy>& plain, Can&& can)
 {
     size_t total = 0;
     for (const Copy& c : copies) total += c.bytes;
@@ -273,7 +274,10 @@ void split_copies(const std::vector<Copy>& copies, std::vector<Copy>& ring, std:
             if (r) total += c.bytes;
         }
     }
-    if (total >= kRingBytes) return;
+    if (total >= kRingBytes) {
+        if (staging_ensure(ctx) == cudaSuccess) return;
+        cudaGetLastError();
+    }
     ring.clear();
     plain = copies;
 }
@@ -283,11 +287,7 @@ void split_copies(const std::vector<Copy>& copies, std::vector<Copy>& ring, std:
 cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies)
 {
     std::vector<InCopy> ring, plain;
-    split_copies(copies, ring, plain, [](const InCopy& c) { return is_pageable(c.src_host); });
-    if (!ring.empty()) {
-        const cudaError_t e = staging_ensure(ctx);
-        if (e != cudaSuccess) return e;
-    }
+    split_copies(ctx, copies, ring, plain, [](const InCopy& c) { return is_pageable(c.src_host); });
     for (const InCopy& c : plain) {
         const cudaError_t e = cudaMemcpyAsync(c.dst_dev, c.src_host, c.bytes, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return e;
@@ -303,7 +303,7 @@ cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>
 {
     // sums are added by the host wherever they lie
     std::vector<OutCopy> ring, plain;
-    split_copies(copies, ring, plain, [](const OutCopy& c) { return c.add || is_pageable(c.dst_host); });
+    split_copies(ctx, copies, ring, plain, [](const OutCopy& c) { return c.add || is_pageable(c.dst_host); });
     size_t added = 0;
     for (const OutCopy& c : plain)
         if (c.add) added += c.bytes / sizeof(double);

@@ -60,6 +60,9 @@ int main()
     round_trip("pageable", 20 * kMiB, {page, page});
     round_trip("locked", 20 * kMiB, {locked, locked, page});
     round_trip("locked_small_rest", 7 * kMiB, {locked, managed, page});
+    g_no_pinned = true;
+    round_trip("no_ring", 20 * kMiB, {page, locked, page});
+    g_no_pinned = false;
     {
         // memory of a device where host memory belongs: an error, and the host never touches it
         fm_ctx ctx;

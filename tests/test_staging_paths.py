@@ -51,6 +51,10 @@ def test_device_memory_in_place_of_host_memory_is_an_error(lines):
     assert [int(v) for v in lines["device"]] == [INVALID_VALUE, INVALID_VALUE]
 
 
+def test_without_page_locked_memory_for_the_ring_the_copies_are_plain(lines):
+    assert _trip(lines, "no_ring") == ((3, 0), (3, 0))
+
+
 @pytest.mark.gpu
 def test_page_locked_arrays_give_the_same_results(ctx):
     import torch
