@@ -8,6 +8,7 @@
 #include <functional>
 #include <mutex>
 #include <new>
+#include <system_error>
 #include <thread>
 
 #include "fm_internal.h"
@@ -19,7 +20,12 @@ class CopyPool {
 public:
     explicit CopyPool(int workers)
     {
-        for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { loop(); });
+        // as many as the system grants: the caller takes part in every round, alone if need be
+        try {
+            for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { loop(); });
+        } catch (const std::system_error&) {
+        } catch (const std::bad_alloc&) {
+        }
     }
     ~CopyPool()
     {

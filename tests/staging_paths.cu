@@ -60,6 +60,11 @@ int main()
     round_trip("pageable", 20 * kMiB, {page, page});
     round_trip("locked", 20 * kMiB, {locked, locked, page});
     round_trip("locked_small_rest", 7 * kMiB, {locked, managed, page});
+    for (int threads : {0, 2}) {
+        g_threads_left = threads;
+        round_trip(threads == 0 ? "no_threads" : "two_threads", 20 * kMiB, {page, page});
+    }
+    g_threads_left = 1 << 30;
     g_no_pinned = true;
     round_trip("no_ring", 20 * kMiB, {page, locked, page});
     g_no_pinned = false;

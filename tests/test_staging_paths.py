@@ -55,6 +55,11 @@ def test_without_page_locked_memory_for_the_ring_the_copies_are_plain(lines):
     assert _trip(lines, "no_ring") == ((3, 0), (3, 0))
 
 
+@pytest.mark.parametrize("name", ["no_threads", "two_threads"])
+def test_fewer_copy_threads_than_asked_for(lines, name):
+    assert _trip(lines, name) == ((0, 1), (0, 1))
+
+
 @pytest.mark.gpu
 def test_page_locked_arrays_give_the_same_results(ctx):
     import torch
