@@ -63,7 +63,7 @@ constexpr int kQcCont = 0 * kQcLine, kQcMis = 1 * kQcLine, kQcShadow = 2 * kQcLi
 constexpr int kQcSet = 3 * kQcLine;
 constexpr int kQcActive = 6 * kQcLine, kQcDisney = 7 * kQcLine, kQcSimple = 8 * kQcLine;
 constexpr int kQcTraceNext = 9 * kQcLine, kQcDisneyR = 10 * kQcLine, kQcSimpleR = 11 * kQcLine;
-constexpr int kQcGrad = 12 * kQcLine, kQcBodies = 13 * kQcLine;
+constexpr int kQcGrad = 12 * kQcLine, kQcBodies = 13 * kQcLine, kQcLimit = 14 * kQcLine;
 constexpr int kQcCount = 16 * kQcLine;
 
 // Records of queued MIS and shadow rays.
@@ -457,6 +457,14 @@ __global__ void k_wf_continue(WfState st, cudaGraphConditionalHandle handle, uns
     const bool overflow = (*(volatile uint32_t*)st.status & 2u) != 0u;
     if (active != 0u && !overflow && bodies >= max_bodies) atomicOr(st.status, 4u);
     cudaGraphSetConditional(handle, (active != 0u && !overflow && bodies < max_bodies) ? 1u : 0u);
+}
+
+// After the iteration at which a caller's limit falls inside a graph body: the body's nth run
+// reports the limit if a slot still holds work there.
+__global__ void k_wf_limit(WfState st, unsigned nth)
+{
+    if (++st.qc[kQcLimit] != nth || st.qc[kQcActive] == 0u) return;
+    if ((*(volatile uint32_t*)st.status & 2u) == 0u) atomicOr(st.status, 4u);
 }
 
 // Rays of the current iteration, [cont | MIS | shadow].  A queue that overflowed counted
@@ -1387,7 +1395,7 @@ struct WfCache {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     WfState g_st;
-    int64_t g_pool = 0, g_max_launches = 0;
+    int64_t g_pool = 0, g_max_bodies = 0, g_limit = 0;
     int g_trace_block = 0, g_shade_block = 0, g_iters = 0;
     bool g_profile = false;
     WfCache()
@@ -1780,9 +1788,18 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     }
     const double iter_bound =
         (z.samples / (double)pool + 4.0 * max_chunk + 8.0) * (max_depth + 2) * 4.0 * (ADJ ? 2.0 : 1.0) + 1000.0;
-    int64_t max_launches = (int64_t)(iter_bound / body_iters) + 16;
-    if (tune.max_iterations > 0)
-        max_launches = std::min<int64_t>(max_launches, (tune.max_iterations + body_iters - 1) / body_iters);
+    // (the host's loop of timed renders sees the end of a body one launch later)
+    int64_t max_bodies = (int64_t)(iter_bound / body_iters) + 16 + (tune.profile ? 1 : 0);
+    // A caller's limit counts whole runs of iters_per_graph iterations, so with an odd number
+    // it can fall inside a body: limit_at is the iteration of the last body that it follows.
+    int64_t limit = 0;
+    int limit_at = 0;
+    if (tune.max_iterations > 0) {
+        const int64_t runs = ((int64_t)tune.max_iterations + tune.iters_per_graph - 1) / tune.iters_per_graph;
+        limit = (runs + (tune.profile ? 1 : 0)) * tune.iters_per_graph;
+        limit_at = (int)(limit % body_iters);
+        max_bodies = std::min(max_bodies, (limit + body_iters - 1) / body_iters);
+    }
     // optional per-kernel timing: event-record nodes around every trace and shade launch
     std::vector<cudaEvent_t>& pev = c->pev;
     if (tune.profile) {
@@ -1829,6 +1846,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
                 k_wf_logic<ADJ, 1><<<logic_grid, 256, 0, s>>>(x);
             if (ADJ) k_wf_grad_scatter<<<sms * 8, 256, 0, s>>>(x);
             if (tune.profile) cudaEventRecordWithFlags(pev[3 * it + 2], s, cudaEventRecordExternal);
+            if (it + 1 == limit_at) k_wf_limit<<<1, 1, 0, s>>>(x, (unsigned)std::min<int64_t>(max_bodies, 0x7fffffff));
         }
     };
     cudaError_t e = cudaSuccess;
@@ -1838,7 +1856,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     const bool reuse = c->exec && std::memcmp(&c->g_st, &st, sizeof(st)) == 0 && c->g_pool == tune.pool &&
                        c->g_trace_block == tune.trace_block && c->g_shade_block == tune.shade_block &&
                        c->g_iters == body_iters && c->g_profile == tune.profile &&
-                       c->g_max_launches == max_launches;
+                       c->g_max_bodies == max_bodies && c->g_limit == limit;
     if (!reuse) {
         wf_cache_drop_graph(*c);
         cudaGraph_t graph = nullptr;
@@ -1861,7 +1879,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
                 e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
             if (e == cudaSuccess) {
                 capture_iterations();
-                k_wf_continue<<<1, 1, 0, s>>>(st, handle, (unsigned)std::min<int64_t>(max_launches, 0x7fffffff));
+                k_wf_continue<<<1, 1, 0, s>>>(st, handle, (unsigned)std::min<int64_t>(max_bodies, 0x7fffffff));
                 e = cudaStreamEndCapture(s, &body);
             }
         } else {
@@ -1884,7 +1902,8 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
         c->g_shade_block = tune.shade_block;
         c->g_iters = body_iters;
         c->g_profile = tune.profile;
-        c->g_max_launches = max_launches;
+        c->g_max_bodies = max_bodies;
+        c->g_limit = limit;
     }
     unsigned* h_qc = c->h_qc;
     int64_t graph_launches = 0;
@@ -1910,6 +1929,8 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
             ++graph_launches;
             e = cudaMemcpyAsync(h_qc, st.qc, sizeof(unsigned) * kQcCount, cudaMemcpyDeviceToHost, s);
             if (e != cudaSuccess) break;
+            e = cudaMemcpyAsync(c->h_status, st.status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+            if (e != cudaSuccess) break;
             e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) break;
             for (int it = 0; it < body_iters; ++it) {
@@ -1920,8 +1941,9 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
                 shade_ms += b;
             }
             // done when no slot holds work after the last shade
-            if (h_qc[kQcActive] == 0u) break;
-            if (++guard > max_launches) {
+            const bool limited = (*c->h_status & 4u) != 0u;
+            if (h_qc[kQcActive] == 0u && !limited) break;
+            if (limited || ++guard >= max_bodies) {
                 result = set_error(ctx, FM_ERR_TIMEOUT, "wavefront: iteration limit reached");
                 break;
             }
@@ -1942,7 +1964,7 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, c->e0, c->e1);
     if (times) {
-        times->launches = 2 + graph_launches * ((ADJ ? 9 : 6) * body_iters + (tune.profile ? 0 : 1)) +
+        times->launches = 2 + graph_launches * ((ADJ ? 9 : 6) * body_iters + (tune.profile ? 0 : 1) + (limit_at > 0 ? 1 : 0)) +
                           (int64_t)views.size();
         times->total_ms = ms;
         times->trace_ms = trace_ms;
