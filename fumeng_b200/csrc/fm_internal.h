@@ -27,7 +27,7 @@ struct fm_ctx {
     // wavefront workspaces (forward, adjoint): state buffers, pinned staging and the
     // instantiated graph, kept between renders
     fm::WfCache* wf_cache[2] = {nullptr, nullptr};
-    size_t wf_limit = 0;      // device bytes that a workspace may hold (0: no limit)
+    size_t wf_limit = 0;      // device bytes that a workspace or the denoiser's records may hold (0: no limit)
     int64_t wf_refused = 0;   // fm_render: fewest path slots beyond the default that did not fit (0: none)
     // scene creation: streams that build scenes side by side
     std::vector<cudaStream_t> build_streams;

@@ -2084,8 +2084,8 @@ fm_status launch_wavefront(fm_ctx* ctx, const fm_scene* scene, const DevCamera& 
 
 }  // namespace fm
 
-// Used by tests: bounds the device memory of each of the context's workspaces (0: by the
-// device only), and reports the forward one's device bytes, how often its state was
+// Used by tests: bounds the device memory of each of the context's workspaces and of the
+// denoiser's records (0: by the device only), and reports the forward one's device bytes, how often its state was
 // allocated and whether it has the second set of ray records.
 extern "C" void fm_internal_limit_workspace(fm_ctx* ctx, int64_t bytes)
 {

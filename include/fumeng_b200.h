@@ -362,7 +362,8 @@ typedef struct {
  * FM_POST_DENOISE needs albedo and normal: the reference calls Intel Open Image Denoise
  * there, which is not available; this library runs an edge-avoiding a-trous wavelet
  * filter guided by the same albedo and normal images instead (its output is not
- * OIDN's).  At most 16 steps.  Host buffers unless FM_FLAG_DEVICE_PTRS. */
+ * OIDN's).  The filter works in 80 B of device memory per pixel, or tile by tile in 12 B
+ * where the device has less.  At most 16 steps.  Host buffers unless FM_FLAG_DEVICE_PTRS. */
 fm_status fm_postprocess(fm_ctx* ctx, int32_t width, int32_t height, const fm_post_step* steps, int32_t num_steps,
                          float* rgb, const float* albedo, const float* normal, uint8_t* rgb8, uint8_t* albedo8,
                          uint8_t* normal8, int32_t flags);

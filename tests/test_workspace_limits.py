@@ -181,3 +181,21 @@ def test_albedo_and_normal_sums_are_held_once_they_are_asked_for(fm_lib):
             np.testing.assert_allclose(x[0], want[0], rtol=1e-5, atol=1e-6)
         for k in (1, 2):
             np.testing.assert_allclose(got[k], want[k], rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(1, 1), (40, 3), (3, 200), (513, 129), (1100, 140), (600, 300)])
+def test_denoiser_in_tiles_gives_the_same_image(w, h, fm_lib):
+    """Where 80 B per pixel are refused, the filter runs tile by tile (512 x 128)."""
+    rng = np.random.default_rng(w + h)
+    rgb = rng.gamma(2.0, 0.3, (h, w, 3)).astype(np.float32)
+    rgb[h // 2, w // 2, 0] = np.inf
+    alb = rng.uniform(0.4, 0.6, (h, w, 3)).astype(np.float32)
+    nrm = (rng.normal(size=(h, w, 3)) * 0.2 + np.array([0, 0, 1.0])).astype(np.float32)
+    chain = [(fb.FM_POST_TONEMAP, 1.1), (fb.FM_POST_DENOISE, 0.0), (fb.FM_POST_DENOISE, 0.0)]
+    with _Ctx() as c:
+        want = c.ctx.postprocess(chain, rgb, alb, nrm)
+        c.limit(79)
+        got = c.ctx.postprocess(chain, rgb, alb, nrm)
+    for a, b in zip(want, got):
+        assert np.array_equal(a, b, equal_nan=a.dtype == np.float32)
