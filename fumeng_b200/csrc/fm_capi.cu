@@ -45,6 +45,14 @@ k_trace_short(const QueryRays q, uint32_t n, uint32_t per_warp, uint32_t* status
 
 }  // namespace
 
+// One ray per lane up to as many rays as lanes can be resident, the stream above.  At that line
+// (151,552 rays on 148 SMs) the first form is ahead, as each warp's start and first claim
+// cost the stream 5 to 30 us; it falls behind between 200,000 and 300,000 incoherent rays,
+// where whole warps wait for their slowest ray a second time, and not at all up to 1 M
+// coherent ones.  One ray per lane / stream, us, around a device-pointer call: 20 k
+// triangles, random rays, 100 k 76 / 87, 152 k 85 / 96, 200 k 96 / 97, 300 k 120 / 109, 1 M
+// 284 / 170; 1.3 M triangles, random, 100 k 158 / 182, 152 k 158 / 172, 300 k 185 / 170, 1 M
+// 415 / 256, camera rays 152 k 156 / 180, 300 k 147 / 155, 1 M 183 / 204.
 cudaError_t fm::launch_query(cudaStream_t stream, int num_sms, const QueryRays& q, int64_t n, unsigned* next, uint32_t* status)
 {
     const int64_t warps = (int64_t)num_sms * kQueryBlocksPerSm * (kQueryBlock / 32);

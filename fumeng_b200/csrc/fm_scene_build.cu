@@ -723,8 +723,10 @@ fm_status create_scenes(fm_ctx* ctx, int32_t n, const fm_scene_desc* const* desc
                 }
                 stager.flush();
             };
-            // a large scene's tables are built while its shading data crosses; a small one's
-            // copies go together
+            // A scene larger than the ring has its tables built while its shading data crosses; a
+            // smaller one's copies go together.  Together / split: 42 MiB 4.0 / 3.4 ms, 71 MiB
+            // 7.1 / 6.3, 187 MiB 16.6 / 16.0; 10 to 18 MiB equal within the spread; batches of
+            // 16 and 64 small scenes 8.98 / 9.07 and 27.45 / 27.51.
             const bool split = B.block_bytes > kStageChunk * kStageChunks;
             if (split)
                 stager.flush();

@@ -241,8 +241,8 @@ FM_D int find_view(const WfState& st, int64_t item)
 //   continuation: (L - C_<=k) (df/dp / f + dlog q/dp - dlog pdf_b/dp)
 // pdf_b is the BSDF density the reference reports and q the sampler's true density
 // (they differ for the Disney reflection lobes; see fm_bsdf_grad.cuh); C_<=k is the
-// radiance collected up to and including vertex k.  The first two are scattered by the
-// trace kernel once visibility and the emitter are known; the third is deferred to the
+// radiance collected up to and including vertex k.  The first two are collected by the
+// resolve kernel once visibility and the emitter are known; the third is deferred to the
 // next shaded vertex, where L - C_<=k is known.  Environment texels enter through Le
 // (bilinear taps) and through the light's sampling and reported densities (importance
 // tables normalised per row and over the whole map), handled by scatter_env and
@@ -824,8 +824,8 @@ struct ShadeJob {
     bool sdelta = false, env = false;
 };
 
-// Shading of the slots whose continuation ray hit a surface of material class CLS (the
-// trace kernel queued them): AOVs at the first bounce, next-event estimation (shadow
+// Shading of the slots whose continuation ray hit a surface of material class CLS
+// (k_wf_resolve_cont queued them): AOVs at the first bounce, next-event estimation (shadow
 // rays), the MIS BSDF samples (MIS rays) and the continuation sample with Russian
 // roulette.  Sets kNextCont / kPending so that the logic kernel keeps the slot's
 // sample open.  Each class runs its own kernel, so a warp holds one kind of BSDF and
