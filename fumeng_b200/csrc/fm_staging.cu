@@ -265,40 +265,37 @@ bool is_pageable(const void* p)
     return false;
 }
 
-// The copies that go through the ring: those that can, when they are kRingBytes in all and
-// there is page-locked memory for the ring (plain copies need none).
+// Whether some copies go through the ring: those that can, when they are kRingBytes in all and
+// there is page-locked memory for the ring (plain copies need none).  Splits them from the rest.
 template <class Copy, class Can>
-void split_copies(fm_ctx* ctx, const std::vector<Copy>& copies, std::vector<Copy>& ring, std::vector<Copy>& plain, Can&& can)
+bool split_copies(fm_ctx* ctx, const std::vector<Copy>& copies, std::vector<Copy>& ring, std::vector<Copy>& rest, Can&& can)
 {
     size_t total = 0;
     for (const Copy& c : copies) total += c.bytes;
-    if (total >= kRingBytes) {
-        total = 0;
-        for (const Copy& c : copies) {
-            const bool r = can(c);
-            (r ? ring : plain).push_back(c);
-            if (r) total += c.bytes;
-        }
+    if (total < kRingBytes) return false;
+    total = 0;
+    for (const Copy& c : copies) {
+        const bool r = can(c);
+        (r ? ring : rest).push_back(c);
+        if (r) total += c.bytes;
     }
-    if (total >= kRingBytes) {
-        if (staging_ensure(ctx) == cudaSuccess) return;
-        cudaGetLastError();
-    }
-    ring.clear();
-    plain = copies;
+    if (total < kRingBytes) return false;
+    if (staging_ensure(ctx) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace
 
 cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copies)
 {
-    std::vector<InCopy> ring, plain;
-    split_copies(ctx, copies, ring, plain, [](const InCopy& c) { return is_pageable(c.src_host); });
-    for (const InCopy& c : plain) {
+    std::vector<InCopy> ring, rest;
+    const bool staged = split_copies(ctx, copies, ring, rest, [](const InCopy& c) { return is_pageable(c.src_host); });
+    for (const InCopy& c : staged ? rest : copies) {
         const cudaError_t e = cudaMemcpyAsync(c.dst_dev, c.src_host, c.bytes, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return e;
     }
-    if (ring.empty()) return cudaSuccess;
+    if (!staged) return cudaSuccess;
     Stager stager(ctx, s);
     for (const InCopy& c : ring) stager.put(c.dst_dev, c.src_host, c.bytes);
     stager.close();
@@ -308,8 +305,9 @@ cudaError_t copy_in(fm_ctx* ctx, cudaStream_t s, const std::vector<InCopy>& copi
 cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>& copies)
 {
     // sums are added by the host wherever they lie
-    std::vector<OutCopy> ring, plain;
-    split_copies(ctx, copies, ring, plain, [](const OutCopy& c) { return c.add || is_pageable(c.dst_host); });
+    std::vector<OutCopy> ring, rest;
+    const bool staged = split_copies(ctx, copies, ring, rest, [](const OutCopy& c) { return c.add || is_pageable(c.dst_host); });
+    const std::vector<OutCopy>& plain = staged ? rest : copies;
     size_t added = 0;
     for (const OutCopy& c : plain)
         if (c.add) added += c.bytes / sizeof(double);
@@ -324,7 +322,7 @@ cudaError_t copy_results(fm_ctx* ctx, cudaStream_t s, const std::vector<OutCopy>
         const cudaError_t e = cudaMemcpyAsync(dst, c.src_dev, c.bytes, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return e;
     }
-    if (!ring.empty()) return copy_out(ctx, s, ring);
+    if (staged) return copy_out(ctx, s, ring);
     if (added == 0) return cudaSuccess;
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
