@@ -1797,8 +1797,11 @@ fm_status run_wavefront(fm_ctx* ctx, const std::vector<WfView>& views_in, const 
     if (tune.max_iterations > 0) {
         const int64_t runs = ((int64_t)tune.max_iterations + tune.iters_per_graph - 1) / tune.iters_per_graph;
         limit = (runs + (tune.profile ? 1 : 0)) * tune.iters_per_graph;
-        limit_at = (int)(limit % body_iters);
-        max_bodies = std::min(max_bodies, (limit + body_iters - 1) / body_iters);
+        const int64_t bodies = (limit + body_iters - 1) / body_iters;
+        if (bodies <= max_bodies) {
+            max_bodies = bodies;
+            limit_at = (int)(limit % body_iters);
+        }
     }
     // optional per-kernel timing: event-record nodes around every trace and shade launch
     std::vector<cudaEvent_t>& pev = c->pev;
